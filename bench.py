@@ -512,9 +512,8 @@ def run_ours(args, world, rank, local):
                    "sample": f"first {ncpu} of {n} samples ({st} cone samples, {dt:.1f} s) traced by the FP32 C++ "
                              "restatement on the same clipmap"}
         # kernels launched per trace step: Morton keys, cub radix sort of 30 bits (histogram, exclusive sum,
-        # 4 onesweep passes), specular keys, cub radix pass on 1 bit (histogram, exclusive sum, onesweep),
-        # diffuse, specular (the texture refresh is a memcpy, not a kernel)
-        launches = 1 if tex is None else 13
+        # 4 onesweep passes), specular list, diffuse, specular (the texture refresh is a memcpy, not a kernel)
+        launches = 1 if tex is None else 10
         line = {
             "metric": METRIC, "value": value, "unit": "cone samples/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
@@ -556,7 +555,7 @@ def run_ours(args, world, rank, local):
                          "frac": achieved / peak, "traffic": traffic,
                          "note": f"{bpcs} B of algorithmic texel reads per cone sample over the {peak_kind} HBM "
                                  "copy peak, per trace step (CUDA events around the step: Morton sort, specular "
-                                 "partition, diffuse and specular kernels; the specular kernel is about 71 % of it "
+                                 "list, diffuse and specular kernels; the specular kernel is about 71 % of it "
                                  "in the ncu launch list); the taps are served mostly from L1/TEX and L2, so the "
                                  "figure exceeds the HBM peak; traffic = ncu DRAM bytes of one step"},
             "gather_roofline": None if gather_peak is None else {
@@ -565,7 +564,7 @@ def run_ours(args, world, rank, local):
                 "frac": cone_samples / (statistics.mean(per) * 1e-3) / gather_peak,
                 "note": "peak = vct_gather_probe: the texture fetches of one cone sample (3 faces x 2 levels, "
                         "trilinear) per step of warp-coherent synthetic cones, measured on this GPU with the same "
-                        "texture; achieved = the whole trace step (Morton sort, specular partition, diffuse and "
+                        "texture; achieved = the whole trace step (Morton sort, specular list, diffuse and "
                         "specular kernels)"},
             "cpu_baseline": cpu,
             "e2e": {"value": total_cone_samples / (e2e_ms * 1e-3), "unit": "cone samples/s",

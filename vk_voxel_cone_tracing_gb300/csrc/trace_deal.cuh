@@ -3,8 +3,8 @@
 // (trace_fast.cu) and the exact FP32 forms (trace_exact.cu), generic in how
 // one cone is marched.
 //
-// The (sample, cone) pairs with cos >= 0 of the warp's 32 samples are dealt
-// to the 32 lanes in rounds, cone-major (lane k of a round takes the k-th
+// The (sample, cone) pairs with cos >= 0 of the warp's samples (up to 32) are
+// dealt to the 32 lanes in rounds, cone-major (lane k of a round takes the k-th
 // pair ordered by cone, then by sample), so no lane idles on a back-facing
 // cone and neighbouring lanes march the same direction from neighbouring
 // samples.  Every sample's cone results are summed by its owner lane in cone
@@ -30,9 +30,28 @@ struct DealArgs {
     int ncones;
     bool need_diffuse;   // trace the diffuse cones (otherwise their sum stays (0, 0, 0, 1))
     bool need_specular;  // specular samples get their specular output from the specular kernel
+    int per_warp = 32;   // samples of one warp item (deal_samples_per_warp); divides 32
 };
 
-// The 32 positions base .. base + 31 of the order on the calling warp.
+// Samples of one warp item: 32, or fewer (down to 4, one round of 16-cone
+// samples) while the items are fewer than `warps`.  An item of 32 marches its
+// cones in about 8 rounds (16 cones, half of them facing away) one after the
+// other, so a trace of few samples leaves most of the chip without a warp;
+// smaller items cost more issue slots in the set-up and the lighting, which
+// run on per_warp lanes.  Measured (R = 128 hall, whole texture trace, us at
+// 32 / 16 / 8 / 4 samples per item): 4096 samples 115 / 74 / 70 / 67, 16,384
+// samples 171 / 146 / 149 / 153, 65,536 samples 316 / 325 / 337 / 352; so the
+// texture form fills 6 warps per SM (its specular kernel runs beside it).  The
+// exact form alone on the chip: 65,536 samples 3344 / 3151 / 3127 / 3189,
+// 131,072 samples 4241 / 4146 / 4226 / 4387, 262,144 samples 6272 / 6389 /
+// 6751: 32 warps per SM.
+inline int deal_samples_per_warp(int64_t n, int64_t warps) {
+    int s = 32;
+    while (s > 4 && (n + s - 1) / s < warps) s >>= 1;
+    return s;
+}
+
+// The positions base .. base + per_warp - 1 of the order on the calling warp.
 // `march(start, dir, start_level, steps)` traces one diffuse cone from `start`
 // and returns traceCone's (rgb, 1 - occlusion).  WARPS = warps per block.
 template <int WARPS, class Marcher>
@@ -49,7 +68,7 @@ __device__ __forceinline__ void deal_diffuse_warp(const DealArgs& A, const March
     const bool c32 = A.ncones == 32;
     {
         const int64_t pos = base + lane;
-        bool valid = pos < A.n;
+        bool valid = lane < A.per_warp && pos < A.n;
         const uint32_t idx = valid ? __ldg(A.order + pos) - A.order_base : 0u;
         valid = valid && idx < A.count;
         GSample g;
@@ -147,7 +166,7 @@ __device__ __forceinline__ void deal_diffuse_warp(const DealArgs& A, const March
     }
 }
 
-// Every warp of the grid over the order, 32 positions at a time: with
+// Every warp of the grid over the order, per_warp positions at a time: with
 // TICKET (`ticket` zeroed before the launch), the items go to the warps as
 // they free up; without, by a static grid stride.
 template <int WARPS, bool TICKET = false, class Marcher>
@@ -159,14 +178,15 @@ __device__ __forceinline__ void deal_diffuse(const DealArgs& A, const Marcher& m
             uint32_t it = 0;
             if (lane == 0) it = atomicAdd(ticket, 1u);
             it = __shfl_sync(0xffffffffu, it, 0);
-            const int64_t base = (int64_t)it * 32;
+            const int64_t base = (int64_t)it * A.per_warp;
             if (base >= A.n) break;
             deal_diffuse_warp<WARPS>(A, march, base, steps);
         }
         return;
     }
     const int64_t nwarps = (int64_t)gridDim.x * WARPS;
-    for (int64_t base = ((int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5)) * 32; base < A.n; base += nwarps * 32)
+    for (int64_t base = ((int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5)) * A.per_warp; base < A.n;
+         base += nwarps * A.per_warp)
         deal_diffuse_warp<WARPS>(A, march, base, steps);
 }
 

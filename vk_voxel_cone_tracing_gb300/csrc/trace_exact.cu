@@ -22,6 +22,7 @@
 namespace vct {
 
 constexpr int kExactWarps = 4;  // warps per block of the diffuse kernel
+constexpr int kExactDiffuseWarpsPerSm = 32;  // warp items per SM that deal_samples_per_warp aims at
 
 // Tickets (work to warps as they free up) for the texture and float reads;
 // the linear RGBA8 atlas's loads run faster with the static deal.
@@ -45,9 +46,9 @@ __global__ void __launch_bounds__(32 * kExactWarps) k_exact_diffuse(TraceParams 
                                                                     int64_t n, const uint32_t* __restrict__ order,
                                                                     float* __restrict__ dout, float* __restrict__ sout,
                                                                     unsigned long long* __restrict__ step_counter,
-                                                                    unsigned int* __restrict__ ticket) {
+                                                                    unsigned int* __restrict__ ticket, int per_warp) {
     const bool c32 = P.d.enable_32_cones != 0;
-    DealArgs D{&P, samples, n, order, 0u, (uint32_t)n, dout, sout, c32 ? 32 : 16, true, true};
+    DealArgs D{&P, samples, n, order, 0u, (uint32_t)n, dout, sout, c32 ? 32 : 16, true, true, per_warp};
     const ExactDiffuseMarch<Atlas> march{T, &P.d, P.diffuse_aperture,
                                          fmaxf(kMinTraceStepFactor, P.d.min_trace_step_factor)};
     unsigned long long steps = 0;
@@ -333,9 +334,10 @@ static int launch_exact(const TraceParams& P, const Atlas& T, const vct_surface_
         if (rc != VCT_OK) return rc;
         unsigned int* spec_ticket = plan.spec_count + 1;
         unsigned int* diff_ticket = plan.spec_count + 2;
-        const int64_t gdw = (m + 32 * kExactWarps - 1) / (32 * kExactWarps);
+        const int per_warp = deal_samples_per_warp(m, 152 * kExactDiffuseWarpsPerSm);
+        const int64_t gdw = (m + (int64_t)per_warp * kExactWarps - 1) / ((int64_t)per_warp * kExactWarps);
         k_exact_diffuse<<<(int)(gdw > 152 * 16 ? 152 * 16 : gdw), 32 * kExactWarps, 0, st>>>(
-            P, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket);
+            P, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
             const int64_t gl = (m + 127) / 128;

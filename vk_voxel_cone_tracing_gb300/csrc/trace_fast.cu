@@ -177,25 +177,66 @@ __device__ __forceinline__ bool traces_specular(const vct_surface_sample* __rest
     return a.w != 1.0f && (d.x > 1e-6f || d.y > 1e-6f || d.z > 1e-6f) && d.w > 1e-6f;
 }
 
-// Specular classification of the Morton-ordered samples (the shader traces
-// a specular cone where depth != 1 and the sample has a specular colour and
-// metalness): key 0 for specular samples, 256 otherwise, and their count.
-// One radix pass on bit 8 then lists the specular samples in Morton order.
-__global__ void k_spec_keys(const __grid_constant__ FastArgs A, const uint32_t* __restrict__ order,
-                            uint32_t* __restrict__ spec_key, unsigned int* __restrict__ spec_count) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < A.n;
-         base += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = base + lane;
-        bool spec = false;
-        if (pos < A.n && A.C.need_specular) spec = traces_specular(A.samples + __ldg(order + pos));
-        if (pos < A.n) spec_key[pos] = spec ? 0u : 256u;
-        const unsigned bal = __ballot_sync(0xffffffffu, spec);
-        if (lane == 0 && bal) atomicAdd(spec_count, (unsigned)__popc(bal));
+// The list of the Morton-ordered samples that trace a specular cone, and its
+// length: a block takes 1024 positions of the order at a time, keeps their
+// order in its piece of the list (ballots, a prefix over its warps) and
+// reserves the piece with one atomic.  Pieces follow one another in the order
+// their blocks arrive, so the list is Morton-ordered but for neighbouring
+// pieces changing places, and a cone's result does not depend on its place.
+// It is bound by the samples' 160-byte reads in that order.
+// `spec_at(pos, &value)`: whether position pos (within range) is listed, and its entry.
+constexpr int kSpecListBlock = 256, kSpecListItems = 4;
+constexpr int kSpecListChunk = kSpecListBlock * kSpecListItems;
+
+template <class SpecAt>
+__device__ __forceinline__ void list_specular(int64_t n, uint32_t* __restrict__ list,
+                                              unsigned int* __restrict__ spec_count, const SpecAt& spec_at) {
+    __shared__ uint32_t s_total[kSpecListBlock / 32], s_base;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t b0 = (int64_t)blockIdx.x * kSpecListChunk; b0 < n; b0 += (int64_t)gridDim.x * kSpecListChunk) {
+        uint32_t value[kSpecListItems], bal[kSpecListItems], total = 0;
+#pragma unroll
+        for (int k = 0; k < kSpecListItems; ++k) {
+            const int64_t pos = b0 + (w * kSpecListItems + k) * 32 + lane;
+            value[k] = 0u;
+            bal[k] = __ballot_sync(0xffffffffu, pos < n && spec_at(pos, value[k]));
+            total += (uint32_t)__popc(bal[k]);
+        }
+        if (lane == 0) s_total[w] = total;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (int i = 0; i < kSpecListBlock / 32; ++i) {
+                const uint32_t c = s_total[i];
+                s_total[i] = sum;
+                sum += c;
+            }
+            s_base = sum ? atomicAdd(spec_count, sum) : 0u;
+        }
+        __syncthreads();
+        uint32_t at = s_base + s_total[w];
+#pragma unroll
+        for (int k = 0; k < kSpecListItems; ++k) {
+            if ((bal[k] >> lane) & 1u) list[at + (uint32_t)__popc(bal[k] & ((1u << lane) - 1u))] = value[k];
+            at += (uint32_t)__popc(bal[k]);
+        }
+        __syncthreads();  // s_total and s_base are rewritten by the next chunk
     }
 }
 
+__global__ void __launch_bounds__(kSpecListBlock) k_spec_list(const __grid_constant__ FastArgs A,
+                                                              const uint32_t* __restrict__ order,
+                                                              uint32_t* __restrict__ list,
+                                                              unsigned int* __restrict__ spec_count) {
+    list_specular(A.n, list, spec_count, [&](int64_t pos, uint32_t& v) {
+        v = __ldg(order + pos);
+        return traces_specular(A.samples + v);
+    });
+}
+
 constexpr int kWarpsPerBlock = 8;
+constexpr int kDiffuseWarpsPerSm = 6;  // warp items per SM that deal_samples_per_warp aims at
 
 // Run the specular cones on a second stream beside the diffuse kernel.
 constexpr bool kTraceSideStream = true;
@@ -217,9 +258,9 @@ struct FastDiffuseMarch {
 };
 
 __global__ void __launch_bounds__(256) k_trace_diffuse(const __grid_constant__ FastArgs A, const uint32_t* __restrict__ order,
-                                                       unsigned int* __restrict__ ticket) {
+                                                       unsigned int* __restrict__ ticket, int per_warp) {
     DealArgs D{&A.P, A.samples, A.n, order, 0u, (uint32_t)A.n, A.dout, A.sout, A.C.ncones, A.C.need_diffuse != 0,
-               A.C.need_specular != 0};
+               A.C.need_specular != 0, per_warp};
     unsigned long long steps = 0;
     // (a ticket for the diffuse items measured no faster than the static stride: 8.69 against 8.66 ms per step)
     deal_diffuse<kWarpsPerBlock, kDiffuseTickets>(D, FastDiffuseMarch{A.tex, &A.C}, steps, ticket);
@@ -454,8 +495,8 @@ struct BatchTable {
     uint32_t bases[kBatchJobs + 1];
     BatchJob jobs[kBatchJobs];
 };
-// kernel parameters may take 32,764 bytes (CUDA 12.1+, compute capability 7.0+); the kernels add at most 24
-static_assert(sizeof(BatchTable) + 24 <= 32764, "the batch table must fit the kernel parameter space");
+// kernel parameters may take 32,764 bytes (CUDA 12.1+, compute capability 7.0+); the kernels add at most 32
+static_assert(sizeof(BatchTable) + 32 <= 32764, "the batch table must fit the kernel parameter space");
 
 // Lane 0's value on every lane.  The batched kernels pass their job index
 // through it: with a job index the compiler cannot prove warp-uniform, the
@@ -487,34 +528,28 @@ __global__ void k_batch_keys(const __grid_constant__ BatchTable T, uint32_t tota
     }
 }
 
-__global__ void k_batch_spec_keys(const __grid_constant__ BatchTable T, uint32_t total,
-                                  const uint32_t* __restrict__ order, uint32_t* __restrict__ spec_key,
-                                  unsigned int* __restrict__ spec_count) {
-    const int lane = threadIdx.x & 31;
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x - lane; b < total; b += gridDim.x * blockDim.x) {
-        const uint32_t pos = b + lane;
-        bool spec = false;
-        if (pos < total) {
-            const uint32_t g = __ldg(order + pos);
-            const BatchJob& J = T.jobs[batch_job_of(T, g)];
-            const uint32_t i = g - J.base;
-            spec = i < J.count && J.A.C.need_specular && traces_specular(J.A.samples + i);
-            spec_key[pos] = spec ? 0u : 256u;
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, spec);
-        if (lane == 0 && bal) atomicAdd(spec_count, (unsigned)__popc(bal));
-    }
+__global__ void __launch_bounds__(kSpecListBlock) k_batch_spec_list(const __grid_constant__ BatchTable T,
+                                                                    uint32_t total,
+                                                                    const uint32_t* __restrict__ order,
+                                                                    uint32_t* __restrict__ list,
+                                                                    unsigned int* __restrict__ spec_count) {
+    list_specular((int64_t)total, list, spec_count, [&](int64_t pos, uint32_t& v) {
+        v = __ldg(order + pos);
+        const BatchJob& J = T.jobs[batch_job_of(T, v)];
+        const uint32_t i = v - J.base;
+        return i < J.count && J.A.C.need_specular && traces_specular(J.A.samples + i);
+    });
 }
 
 __global__ void __launch_bounds__(256) k_batch_diffuse(const __grid_constant__ BatchTable T, uint32_t total,
-                                                       const uint32_t* __restrict__ order) {
+                                                       const uint32_t* __restrict__ order, int per_warp) {
     const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    for (int64_t base = ((int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5)) * 32; base < total;
-         base += nwarps * 32) {
+    for (int64_t base = ((int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5)) * per_warp; base < total;
+         base += nwarps * per_warp) {
         const BatchJob& J = T.jobs[warp_uniform(batch_job_of(T, (uint32_t)base))];  // 32-aligned segments: one job
         const FastArgs& A = J.A;
         DealArgs D{&A.P, A.samples, (int64_t)total, order, J.base, J.count, A.dout, A.sout, A.C.ncones,
-                   A.C.need_diffuse != 0, A.C.need_specular != 0};
+                   A.C.need_diffuse != 0, A.C.need_specular != 0, per_warp};
         unsigned long long steps = 0;
         deal_diffuse_warp<kWarpsPerBlock>(D, FastDiffuseMarch{A.tex, &A.C}, base, steps);
         add_steps(A.steps, steps);
@@ -598,7 +633,7 @@ __global__ void __launch_bounds__(256) k_gather_probe(const __grid_constant__ Fa
 
 // ------------------------------------------------------------- scratch layout
 struct FastScratch {
-    uint32_t *keys_in, *keys_out, *vals_in, *order, *spec_key, *spec_key_out, *spec_list;
+    uint32_t *keys_in, *keys_out, *vals_in, *order, *spec_list;
     unsigned int* spec_count;
     void* temp;
     size_t temp_bytes;
@@ -608,12 +643,9 @@ struct FastScratch {
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 static int plan_scratch(int64_t n, void* base, FastScratch& s) {
-    size_t t1 = 0, t2 = 0;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, t1, (uint32_t*)nullptr, (uint32_t*)nullptr,
+    size_t temp_bytes = 0;
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                                     (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, 0, 30);
-    if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
-    e = cub::DeviceRadixSort::SortPairs(nullptr, t2, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                        (uint32_t*)nullptr, (int)n, 0, 9);
     if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
     const size_t arr = align256(sizeof(uint32_t) * (size_t)n);
     char* p = (char*)base;
@@ -627,11 +659,9 @@ static int plan_scratch(int64_t n, void* base, FastScratch& s) {
     s.keys_out = (uint32_t*)take(arr);
     s.vals_in = (uint32_t*)take(arr);
     s.order = (uint32_t*)take(arr);
-    s.spec_key = (uint32_t*)take(arr);
-    s.spec_key_out = (uint32_t*)take(arr);
     s.spec_list = (uint32_t*)take(arr);
     s.spec_count = (unsigned int*)take(256);
-    s.temp_bytes = t1 > t2 ? t1 : t2;
+    s.temp_bytes = temp_bytes;
     s.temp = take(s.temp_bytes);
     s.total = off;
     return VCT_OK;
@@ -768,7 +798,7 @@ FastShape fast_shape(int R) {
 }
 
 // The trace pipeline after argument checks: Morton keys and sort, specular
-// classification and partition, the diffuse and specular kernels.
+// list, the diffuse and specular kernels.
 int launch_fast(const FastArgs& A, const FastScratch& S, int64_t n, FastShape sh, cudaStream_t st) {
     const int sms = sm_count();
     const int block = 256;
@@ -780,16 +810,18 @@ int launch_fast(const FastArgs& A, const FastScratch& S, int64_t n, FastShape sh
     VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(S.temp, tb, S.keys_in, S.keys_out, S.vals_in, S.order, (int)n, 0, 30, st));
     // the specular count and the tickets of the specular cones and the diffuse items
     VCT_CUDA_TRY(cudaMemsetAsync(S.spec_count, 0, 3 * sizeof(unsigned int), st));
-    int64_t gd = (n + 255) / 256;
+    const int per_warp = deal_samples_per_warp(n, (int64_t)sms * kDiffuseWarpsPerSm);
+    int64_t gd = (n + (int64_t)per_warp * kWarpsPerBlock - 1) / ((int64_t)per_warp * kWarpsPerBlock);
     const int64_t cap_d = (int64_t)sms * sh.diffuse_per_sm;
     const int grid_d = (int)(gd > cap_d ? cap_d : gd);
     if (!A.C.need_specular) {
-        k_trace_diffuse<<<grid_d, 256, 0, st>>>(A, S.order, S.spec_count + 2);
+        k_trace_diffuse<<<grid_d, 256, 0, st>>>(A, S.order, S.spec_count + 2, per_warp);
         VCT_LAUNCH_CHECK();
         return VCT_OK;
     }
-    const int grid_k = (int)(gd > (int64_t)sms * 16 ? (int64_t)sms * 16 : gd);
-    // the specular classification, partition and cones on the second stream,
+    const int64_t gk = (n + kSpecListChunk - 1) / kSpecListChunk;
+    const int grid_k = (int)(gk > (int64_t)sms * 8 ? (int64_t)sms * 8 : gk);
+    // the specular list and cones on the second stream,
     // beside the diffuse kernel (they share only the sorted order, read-only)
     TraceSide* side = kTraceSideStream ? trace_side() : nullptr;
     cudaStream_t ss = side ? side->s : st;
@@ -797,18 +829,14 @@ int launch_fast(const FastArgs& A, const FastScratch& S, int64_t n, FastShape sh
         VCT_CUDA_TRY(cudaEventRecord(side->fork, st));
         VCT_CUDA_TRY(cudaStreamWaitEvent(ss, side->fork, 0));
     }
-    k_spec_keys<<<grid_k, 256, 0, ss>>>(A, S.order, S.spec_key, S.spec_count);
+    k_spec_list<<<grid_k, kSpecListBlock, 0, ss>>>(A, S.order, S.spec_list, S.spec_count);
     VCT_LAUNCH_CHECK();
-    tb = S.temp_bytes;
-    // stable partition (one radix pass on bit 8): specular samples first, Morton order kept
-    VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(S.temp, tb, S.spec_key, S.spec_key_out, S.order, S.spec_list, (int)n,
-                                                 8, 9, ss));
     int64_t gw = (n * 32 + 255) / 256;
     const int64_t cap_s = (int64_t)sms * sh.specular_per_sm;
     const int grid_s = (int)(gw > cap_s ? cap_s : gw);
     k_trace_specular_warp<<<grid_s, 256, 0, ss>>>(A, S.spec_list, S.spec_count, S.spec_count + 1);
     VCT_LAUNCH_CHECK();
-    k_trace_diffuse<<<grid_d, 256, 0, st>>>(A, S.order, S.spec_count + 2);
+    k_trace_diffuse<<<grid_d, 256, 0, st>>>(A, S.order, S.spec_count + 2, per_warp);
     VCT_LAUNCH_CHECK();
     if (side) {
         VCT_CUDA_TRY(cudaEventRecord(side->join, ss));
@@ -979,7 +1007,7 @@ namespace {
 // largest chunk's layout (chunks run one after the other on the stream).
 struct BatchLayout {
     uint32_t positions;  // padded global positions of the largest chunk
-    size_t keys_in, keys_out, vals_in, order, spec_key, spec_key_out, spec_list, spec_count, temp;
+    size_t keys_in, keys_out, vals_in, order, spec_list, spec_count, temp;
     size_t temp_bytes, total;
 };
 
@@ -1002,15 +1030,11 @@ int batch_layout(const vct_trace_job* jobs, int32_t njobs, BatchLayout& L) {
     L.positions = (uint32_t)most;
     int jb = 0;
     while ((1 << jb) < kBatchJobs) ++jb;
-    size_t t1 = 0, t2 = 0;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, t1, (unsigned long long*)nullptr,
+    L.temp_bytes = 0;
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, L.temp_bytes, (unsigned long long*)nullptr,
                                                     (unsigned long long*)nullptr, (uint32_t*)nullptr,
                                                     (uint32_t*)nullptr, (int)L.positions, 0, 31 + jb);
-    if (e == cudaSuccess)
-        e = cub::DeviceRadixSort::SortPairs(nullptr, t2, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                            (uint32_t*)nullptr, (int)L.positions, 8, 9);
     if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
-    L.temp_bytes = t1 > t2 ? t1 : t2;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t at = off;
@@ -1022,8 +1046,6 @@ int batch_layout(const vct_trace_job* jobs, int32_t njobs, BatchLayout& L) {
     L.keys_out = take(8 * n);
     L.vals_in = take(4 * n);
     L.order = take(4 * n);
-    L.spec_key = take(4 * n);
-    L.spec_key_out = take(4 * n);
     L.spec_list = take(4 * n);
     L.spec_count = take(2 * sizeof(unsigned int));
     L.temp = take(L.temp_bytes);
@@ -1072,8 +1094,6 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
     auto* keys_out = reinterpret_cast<unsigned long long*>(b + L.keys_out);
     uint32_t* vals_in = reinterpret_cast<uint32_t*>(b + L.vals_in);
     uint32_t* order = reinterpret_cast<uint32_t*>(b + L.order);
-    uint32_t* spec_key = reinterpret_cast<uint32_t*>(b + L.spec_key);
-    uint32_t* spec_key_out = reinterpret_cast<uint32_t*>(b + L.spec_key_out);
     uint32_t* spec_list = reinterpret_cast<uint32_t*>(b + L.spec_list);
     unsigned int* spec_count = reinterpret_cast<unsigned int*>(b + L.spec_count);
     int jb = 0;
@@ -1116,13 +1136,13 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
         VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(b + L.temp, tb, keys_in, keys_out, vals_in, order, (int)n, 0,
                                                      31 + jb, st));
         VCT_CUDA_TRY(cudaMemsetAsync(spec_count, 0, 2 * sizeof(unsigned int), st));  // count and cone ticket
-        k_batch_spec_keys<<<(g256 > 152 * 16 ? 152 * 16 : g256), 256, 0, st>>>(T, pos, order, spec_key, spec_count);
+        const int64_t gk = (n + kSpecListChunk - 1) / kSpecListChunk;
+        k_batch_spec_list<<<(int)(gk > 152 * 8 ? 152 * 8 : gk), kSpecListBlock, 0, st>>>(T, pos, order, spec_list,
+                                                                                       spec_count);
         VCT_LAUNCH_CHECK();
-        tb = L.temp_bytes;
-        // stable partition (one radix pass on bit 8): specular positions first, the coherent order kept
-        VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(b + L.temp, tb, spec_key, spec_key_out, order, spec_list,
-                                                     (int)n, 8, 9, st));
-        k_batch_diffuse<<<(g256 > 152 * 8 ? 152 * 8 : g256), 256, 0, st>>>(T, pos, order);
+        const int per_warp = deal_samples_per_warp(n, 152 * kDiffuseWarpsPerSm);
+        const int64_t gd = (n + (int64_t)per_warp * kWarpsPerBlock - 1) / ((int64_t)per_warp * kWarpsPerBlock);
+        k_batch_diffuse<<<(int)(gd > 152 * 8 ? 152 * 8 : gd), 256, 0, st>>>(T, pos, order, per_warp);
         VCT_LAUNCH_CHECK();
         const int64_t gw = (n * 32 + 255) / 256;
         k_batch_specular<<<(int)(gw > 152 * 64 ? 152 * 64 : gw), 256, 0, st>>>(T, spec_list, spec_count,
