@@ -4,11 +4,33 @@
 // Same cone loop as the clipmap tracer, sampling the pool by point location:
 // sampleSVO normalises the position by a scene box (the shader hard-codes
 // Sponza's), descends from uVolumeDimension to resolution 2^level and reads
-// the node's RGBA8; two levels are mixed by fract(level).  One thread per
-// G-buffer sample, FP32 in the shader's order (-fmad=false), so the results
-// track the FP32 restatement; the pool descents are dependent loads served
-// from L2 (a depth-8 pool of a few million nodes is L2-resident).
-#include "trace_common.cuh"
+// the node's RGBA8; two levels are mixed by fract(level).  FP32 in the
+// shader's order (-fmad=false), so the results track the FP32 restatement.
+//
+// Work layout: the exact clipmap trace's plan (samples in the coherent order;
+// the diffuse cones of a warp's samples dealt to its lanes, trace_deal.cuh;
+// the specular cones one per lane over a list grouped by aperture), instead
+// of one thread marching a sample's 17 cones.  The march is bound by its own
+// arithmetic (the pool stays in L2, and most of the box is empty space that a
+// descent leaves after a node or two), so each step computes only what its
+// result needs, every needed value being the shader expression's bit for bit:
+//   * both levels' nodes come from one descent (the coarser is an ancestor),
+//     child slots straight from the cell's bits, a node read as one 8 bytes;
+//   * the cell is a fused multiply-add and a floor per axis, the shader's
+//     divisions only where the position is within rounding of a cell border;
+//   * min_level is the exponent of the squared distance, the square root,
+//     division and logarithm only within 2^-16 of a power of two;
+//   * the diffuse cones' level by step comes from a table (the schedule is the
+//     same for all of them);
+//   * a step whose two nodes are zero leaves the composite as it is, so level
+//     size, opacity power and divisions run for the others alone.
+// Measured: the trace of 1,000,003 samples on the 4M-triangle terrain at
+// L = 9 went from 4.9 to 1.4 ms, 65,536 samples on the room at L = 7 from 0.57
+// to 0.42 ms, every output unchanged.
+#include <cmath>
+
+#include "trace_deal.cuh"
+#include "trace_exact.cuh"
 
 namespace vct {
 
@@ -19,116 +41,135 @@ int fill_trace_params(TraceParams& P, const vct_cone_tracing_desc* desc, const v
 struct SvoScene {
     const uint2* __restrict__ pool;
     uint32_t nodes;
-    float bmin[3], bmax[3];
+    uint32_t dim;        // the root resolution, a power of two
+    int top;             // its log2 - 1: the cell bit of the first descent step
+    float c[3], ev;      // box centre and half extent
+    float a, b[3];       // cell coordinate = p * a + b, up to rounding
+    float ga, g0[3];     // bound of that rounding: |p| * ga + g0
+    float min_radius, inv_r2, inv_uvs;
+    bool uvs_pow2;       // voxel_size is a power of two: x * inv_uvs == x / voxel_size
 };
 
-__device__ inline float4 sample_svo(const SvoScene& S, const vct_cone_tracing_desc& d, float3 p, uint32_t level) {
-    const float ex = S.bmax[0] - S.bmin[0], ey = S.bmax[1] - S.bmin[1], ez = S.bmax[2] - S.bmin[2];
-    const float ev = fmaxf(ex, fmaxf(ey, ez)) * 0.5f;
-    const float c[3] = {(S.bmin[0] + S.bmax[0]) * 0.5f, (S.bmin[1] + S.bmax[1]) * 0.5f, (S.bmin[2] + S.bmax[2]) * 0.5f};
-    uint32_t resolution = (uint32_t)d.volume_dimension;
-    const float pp[3] = {p.x, p.y, p.z};
-    uint32_t fp[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float s = (pp[a] - c[a]) / ev;
-        float u = ((s + 1.0f) * 0.5f) * (float)resolution;
-        u = fmaxf(u, 0.0f);
-        const uint32_t q = (uint32_t)fminf(u, 4294967040.0f);
-        fp[a] = min(q, resolution);
+// sampleSVO's cell of coordinate p on axis k, clamped to the last cell (the
+// shader's cell `resolution` takes the upper child at every step, as the last
+// cell does).
+__device__ __forceinline__ uint32_t svo_cell(const SvoScene& S, float p, int k) {
+    const float q = fmaf(p, S.a, S.b[k]), g = fmaf(fabsf(p), S.ga, S.g0[k]);
+    float u = floorf(q);
+    const float r = q - u;
+    if (!(r > g && r < 1.0f - g)) {  // within rounding of a border (or not finite): the shader's expression
+        const float s = (p - S.c[k]) / S.ev;
+        u = ((s + 1.0f) * 0.5f) * (float)S.dim;
     }
-    const uint32_t target = 1u << level;
-    uint32_t idx = 0, cur = 0;
-    do {
-        resolution >>= 1;
-        const uint32_t cx = fp[0] >= resolution, cy = fp[1] >= resolution, cz = fp[2] >= resolution;
-        idx = cur + (cz | (cx << 1) | (cy << 2));
-        if (idx >= S.nodes) return make_float4(0.f, 0.f, 0.f, 0.f);  // malformed pool: never read past it
-        cur = __ldg(&S.pool[idx].x) & 0x7fffffffu;
-        fp[0] -= cx * resolution;
-        fp[1] -= cy * resolution;
-        fp[2] -= cz * resolution;
-    } while (cur != 0u && resolution > target);
-    const uint32_t v = __ldg(&S.pool[idx].y);
-    return unpack_rgba8(v);
+    return min((uint32_t)fminf(fmaxf(u, 0.0f), 4294967040.0f), S.dim - 1u);
 }
 
+// The RGBA8 words of the nodes at levels lo <= hi around p.
+__device__ __forceinline__ uint2 svo_nodes(const SvoScene& S, float3 p, uint32_t lo, uint32_t hi) {
+    const uint32_t x = svo_cell(S, p.x, 0), y = svo_cell(S, p.y, 1), z = svo_cell(S, p.z, 2);
+    const uint32_t target_lo = 1u << lo, target_hi = 1u << hi;
+    uint32_t cur = 0, vlo = 0, vhi = 0;
+    bool coarse = true;  // the coarser node not reached yet
+    int b = S.top;
+    for (;;) {
+        const uint32_t idx = cur + (((z >> b) & 1u) | (((x >> b) & 1u) << 1) | (((y >> b) & 1u) << 2));
+        if (idx >= S.nodes) {  // malformed pool: never read past it, the sample is empty
+            vlo = 0;
+            if (coarse) vhi = 0;
+            break;
+        }
+        const uint2 n = __ldg(S.pool + idx);
+        cur = n.x & 0x7fffffffu;
+        vlo = n.y;
+        if (coarse) {
+            vhi = n.y;
+            coarse = cur != 0u && (1u << b) > target_hi;
+        }
+        if (cur == 0u || (1u << b) <= target_lo) break;
+        --b;
+    }
+    return make_uint2(vlo, vhi);
+}
+
+// ceil(log2(|center - pos| / min_radius)) from the squared distance: with
+// t = (dist / radius)^2 up to a few ulp, ceil(log2(t) / 2) is an exponent
+// unless t is next to an even power of two, where the shader's expression
+// decides (its logarithm is within an ulp, which moves no other ceil).
+__device__ __forceinline__ float svo_min_level(const SvoScene& S, float3 center, float3 pos) {
+    const float d2 = dot3(center - pos, center - pos);
+    const uint32_t bits = __float_as_uint(d2 * S.inv_r2);
+    const int rel = (int)(bits - 0x3f800000u);  // even powers of two are multiples of 2^24
+    if (((uint32_t)(rel + 128) & 0xffffffu) < 256u || bits - 0x0d800000u >= 0x64800000u)
+        return ceilf(log2f(sqrtf(d2) / S.min_radius));
+    return (float)((rel >> 24) + 1);
+}
+
+__device__ __forceinline__ float svo_over_uvs(const SvoScene& S, float x, float uvs) {
+    return S.uvs_pow2 ? x * S.inv_uvs : x / uvs;
+}
+
+// traceCone over the pool.  level_at[k] (k < levels): log2(diameter / uvs) of step k, where the caller has it.
 __device__ float4 svo_trace_cone(const SvoScene& S, const vct_cone_tracing_desc& d, float3 start, float3 dir,
-                                 float aperture, float start_level, float step_factor, unsigned long long& steps) {
+                                 float cone_coef, float start_level, float step_factor, const float* level_at,
+                                 int levels, unsigned long long& steps) {
     float4 result = make_float4(0.f, 0.f, 0.f, 0.f);
     const float uvs = d.voxel_size;
-    const float cone_coef = 2.0f * tanf(aperture * 0.5f);
-    float cur_level = start_level;
-    float vs = uvs * exp2f(cur_level);
+    float vs = uvs * exp2f(start_level);
     start = start + dir * (vs * d.trace_start_offset * 0.5f);
     float step = 0.0f, diameter = fmaxf(step * cone_coef, uvs), occlusion = 0.0f, seg = vs;
-    const float min_radius = uvs * d.volume_dimension * 0.5f;
     const float3 center = f3(d.volume_center[0], d.volume_center[1], d.volume_center[2]);
+    int k = 0;
     while (step < kMaxTraceDistance && occlusion < 1.0f) {
-        ++steps;
         const float3 pos = start + dir * step;
-        const float dist = sqrtf(dot3(center - pos, center - pos));
-        const float min_level = ceilf(log2f(dist / min_radius));
-        cur_level = log2f(diameter / uvs);
+        const float min_level = svo_min_level(S, center, pos);
+        float cur_level;
+        if (k < levels) cur_level = level_at[k];
+        else cur_level = log2f(svo_over_uvs(S, diameter, uvs));
+        ++k;
         cur_level = fminf(fmaxf(fmaxf(start_level, cur_level), min_level), (float)(kClipLevels - 1));
-        const uint32_t lo = (uint32_t)floorf(cur_level), hi = (uint32_t)ceilf(cur_level);
-        const float4 a = sample_svo(S, d, pos, lo), b = sample_svo(S, d, pos, hi);
-        const float fr = fractf(cur_level);
-        const float4 s = make_float4(a.x * (1.0f - fr) + b.x * fr, a.y * (1.0f - fr) + b.y * fr,
-                                     a.z * (1.0f - fr) + b.z * fr, a.w * (1.0f - fr) + b.w * fr);
-        vs = uvs * exp2f(cur_level);
-        const float correction = seg / vs;
-        const float rx = s.x * correction, ry = s.y * correction, rz = s.z * correction;
-        // alpha rounded above 1 (a pow of a negative base, undefined in GLSL) is taken as 1
-        const float opacity = clampf(1.0f - powf(fmaxf(1.0f - s.w, 0.0f), correction), 0.0f, 1.0f);
-        const float k = clampf(1.0f - result.w, 0.0f, 1.0f);
-        result = make_float4(result.x + k * rx, result.y + k * ry, result.z + k * rz, result.w + k * opacity);
-        occlusion = occlusion + (1.0f - occlusion) * opacity / (1.0f + (step + vs) * d.occlusion_decay);
+        const uint2 v = svo_nodes(S, pos, (uint32_t)floorf(cur_level), (uint32_t)ceilf(cur_level));
+        if (v.x | v.y) {
+            const float4 a = unpack_rgba8(v.x), b = unpack_rgba8(v.y);
+            const float fr = fractf(cur_level);
+            const float4 s = make_float4(a.x * (1.0f - fr) + b.x * fr, a.y * (1.0f - fr) + b.y * fr,
+                                         a.z * (1.0f - fr) + b.z * fr, a.w * (1.0f - fr) + b.w * fr);
+            vs = uvs * exp2f(cur_level);
+            const float correction = seg / vs;
+            const float rx = s.x * correction, ry = s.y * correction, rz = s.z * correction;
+            // alpha rounded above 1 (a pow of a negative base, undefined in GLSL) is taken as 1
+            const float opacity = clampf(1.0f - powf(fmaxf(1.0f - s.w, 0.0f), correction), 0.0f, 1.0f);
+            const float q = clampf(1.0f - result.w, 0.0f, 1.0f);
+            result = make_float4(result.x + q * rx, result.y + q * ry, result.z + q * rz, result.w + q * opacity);
+            occlusion = occlusion + (1.0f - occlusion) * opacity / (1.0f + (step + vs) * d.occlusion_decay);
+        }
         const float prev = step;
         step = step + fmaxf(diameter, uvs) * step_factor;
         seg = step - prev;
         diameter = step * cone_coef;
     }
+    steps += (unsigned)k;
     return make_float4(clampf(result.x, 0.f, 1.f), clampf(result.y, 0.f, 1.f), clampf(result.z, 0.f, 1.f),
                        clampf(1.0f - occlusion, 0.f, 1.f));
 }
 
-__global__ void __launch_bounds__(128) k_svo_trace(TraceParams P, SvoScene S, const vct_surface_sample* __restrict__ samples,
-                                                   int64_t n, const uint32_t* __restrict__ order,
-                                                   float* __restrict__ dout, float* __restrict__ sout,
-                                                   unsigned long long* __restrict__ step_counter,
-                                                   unsigned int* __restrict__ ticket) {
-    unsigned long long steps = 0;
-    const vct_cone_tracing_desc& d = P.d;
-    const int lane = threadIdx.x & 31;
-    // 32 consecutive samples of the coherent order per warp, dealt by a ticket as warps free up
-    for (;;) {
-        uint32_t t0 = 0;
-        if (lane == 0) t0 = atomicAdd(ticket, 32u);
-        t0 = __shfl_sync(0xffffffffu, t0, 0);
-        if ((int64_t)t0 >= n) break;
-        const int64_t t = (int64_t)t0 + lane;
-        if (t >= n) continue;
-        const int64_t i = order ? (int64_t)__ldg(order + t) : t;
-        GSample g = load_sample(samples + i, P.eye);
-        if (g.depth == 1.0f) continue;
-        const float min_level = calc_min_level(d, g.wp);
-        const float vs = d.voxel_size * exp2f(min_level);
-        const float3 start = g.wp + g.normal * (vs * d.trace_start_offset);
-        float4 ind = make_float4(0.f, 0.f, 0.f, 1.f);
+// The rendering-mode switch of voxelConeTracing_Octree.frag, its two outputs.
+__device__ __forceinline__ float4 svo_specular_out(uint32_t mode, float3 ispec) {
+    if (mode == 6u || mode >= 8u) return make_float4(0.f + ispec.x, 0.f + ispec.y, 0.f + ispec.z, 1.f);
+    return make_float4(0.f, 0.f, 0.f, 1.f);
+}
+
+struct SvoFinish {
+    const DealArgs& A;
+    __device__ __forceinline__ void operator()(const GSample& g, float min_level, float4 ind, uint32_t idx) const {
+        const TraceParams& P = *A.P;
+        const vct_cone_tracing_desc& d = P.d;
+        const bool c32 = A.ncones == 32;
         float valid = 0.0f;
-        const bool c32 = d.enable_32_cones != 0;
-        const int nc = c32 ? 32 : 16;
-        const float aperture = c32 ? kAperture32 : kAperture16;
-        const float sf = fmaxf(kMinTraceStepFactor, d.min_trace_step_factor);
-        for (int c = 0; c < nc; ++c) {
+        for (int c = 0; c < A.ncones; ++c) {
             const float3 dir = c32 ? f3(c_dirs32[c][0], c_dirs32[c][1], c_dirs32[c][2])
                                    : f3(c_dirs16[c][0], c_dirs16[c][1], c_dirs16[c][2]);
             const float cos_t = dot3(g.normal, dir);
-            if (cos_t < 0.0f) continue;
-            const float4 r = svo_trace_cone(S, d, start, dir, aperture, min_level, sf, steps);
-            ind = make_float4(ind.x + r.x * cos_t, ind.y + r.y * cos_t, ind.z + r.z * cos_t, ind.w + r.w * cos_t);
-            valid = valid + cos_t;
+            if (!(cos_t < 0.0f)) valid = valid + cos_t;
         }
         ind = make_float4(ind.x / valid, ind.y / valid, ind.z / valid, ind.w / valid);
         ind.w = ind.w * d.ambient_occlusion_factor;
@@ -136,17 +177,9 @@ __global__ void __launch_bounds__(128) k_svo_trace(TraceParams P, SvoScene S, co
         ind.y = ind.y * (g.diffuse_color.y * d.indirect_diffuse_intensity);
         ind.z = ind.z * (g.diffuse_color.z * d.indirect_diffuse_intensity);
         ind = make_float4(clampf(ind.x, 0.f, 1.f), clampf(ind.y, 0.f, 1.f), clampf(ind.z, 0.f, 1.f), clampf(ind.w, 0.f, 1.f));
-        float3 ispec = f3(0.f, 0.f, 0.f);
-        if (has_specular_cone(g)) {
-            const float3 sdir = normalize3(reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal));
-            const float4 r = svo_trace_cone(S, d, start, sdir, fmaxf(g.roughness, kMinSpecularAperture), min_level,
-                                            fmaxf(kMinTraceStepFactor, d.voxel_size), steps);
-            const float isi = d.indirect_specular_intensity;
-            ispec = f3(r.x * g.specular_color.x * isi, r.y * g.specular_color.y * isi, r.z * g.specular_color.z * isi);
-        }
         float3 direct = direct_term(P, g);
         direct = f3(clampf(direct.x, 0.f, 1.f), clampf(direct.y, 0.f, 1.f), clampf(direct.z, 0.f, 1.f));
-        float4 D = make_float4(0.f, 0.f, 0.f, 1.f), Sp = make_float4(0.f, 0.f, 0.f, 1.f);
+        float4 D = make_float4(0.f, 0.f, 0.f, 1.f);
         switch (d.rendering_mode) {
             case 0: D = make_float4(g.diffuse_color.x, g.diffuse_color.y, g.diffuse_color.z, 1.f); break;
             case 1: D = make_float4(g.specular_color.x, g.specular_color.y, g.specular_color.z, 1.f); break;
@@ -171,21 +204,104 @@ __global__ void __launch_bounds__(128) k_svo_trace(TraceParams P, SvoScene S, co
                 D = make_float4(direct.x, direct.y, direct.z, 1.f);
                 break;
             case 5: D = make_float4(D.x + ind.x, D.y + ind.y, D.z + ind.z, 1.f); break;
-            case 6: Sp = make_float4(Sp.x + ispec.x, Sp.y + ispec.y, Sp.z + ispec.z, 1.f); break;
+            case 6: break;
             case 7: D = make_float4(ind.w, ind.w, ind.w, 1.f); break;
             default:
                 direct = direct * ind.w;
                 D = make_float4(D.x + direct.x + ind.x, D.y + direct.y + ind.y, D.z + direct.z + ind.z, 1.f);
-                Sp = make_float4(Sp.x + ispec.x, Sp.y + ispec.y, Sp.z + ispec.z, 1.f);
                 break;
         }
-        reinterpret_cast<float4*>(dout)[i] = D;
-        reinterpret_cast<float4*>(sout)[i] = Sp;
+        reinterpret_cast<float4*>(A.dout)[idx] = D;
+        if (!has_specular_cone(g))
+            reinterpret_cast<float4*>(A.sout)[idx] = svo_specular_out(d.rendering_mode, f3(0.f, 0.f, 0.f));
     }
-    if (step_counter) {
-        for (int o = 16; o > 0; o >>= 1) steps += __shfl_xor_sync(0xffffffffu, steps, o);
-        if ((threadIdx.x & 31) == 0 && steps) atomicAdd(step_counter, steps);
+};
+
+constexpr int kSvoWarps = 4;  // warps per block of the diffuse kernel
+constexpr int kSvoWarpsPerSm = 16;  // warp items per SM that deal_samples_per_warp aims at
+constexpr int kSvoLevels = 128;  // steps of the diffuse schedule kept as a table (default descriptors take 19 to 40)
+
+struct SvoDiffuseMarch {
+    const SvoScene* S;
+    const vct_cone_tracing_desc* d;
+    float coef, step_factor;
+    const float* level_at;
+    int levels;
+    __device__ __forceinline__ float4 operator()(float3 start, float3 dir, float start_level,
+                                                 unsigned long long& steps) const {
+        return svo_trace_cone(*S, *d, start, dir, coef, start_level, step_factor, level_at, levels, steps);
     }
+};
+
+__global__ void __launch_bounds__(32 * kSvoWarps) k_svo_diffuse(const __grid_constant__ TraceParams P,
+                                                                const __grid_constant__ SvoScene S,
+                                                                const vct_surface_sample* __restrict__ samples,
+                                                                int64_t n, const uint32_t* __restrict__ order,
+                                                                float* __restrict__ dout, float* __restrict__ sout,
+                                                                unsigned long long* __restrict__ step_counter,
+                                                                unsigned int* __restrict__ ticket, int per_warp) {
+    __shared__ float s_level[kSvoLevels];
+    __shared__ int s_levels;
+    const bool c32 = P.d.enable_32_cones != 0;
+    const float uvs = P.d.voxel_size;
+    const float coef = 2.0f * tanf((c32 ? kAperture32 : kAperture16) * 0.5f);
+    const float sf = fmaxf(kMinTraceStepFactor, P.d.min_trace_step_factor);
+    if (threadIdx.x == 0) {  // the march's own recurrence
+        float step = 0.0f, diameter = fmaxf(step * coef, uvs);
+        int k = 0;
+        for (; k < kSvoLevels && step < kMaxTraceDistance; ++k) {
+            s_level[k] = diameter;
+            step = step + fmaxf(diameter, uvs) * sf;
+            diameter = step * coef;
+        }
+        s_levels = k;
+    }
+    __syncthreads();
+    const int levels = s_levels;
+    for (int k = threadIdx.x; k < levels; k += blockDim.x) s_level[k] = log2f(svo_over_uvs(S, s_level[k], uvs));
+    __syncthreads();
+    DealArgs D{&P, samples, n, order, 0u, (uint32_t)n, dout, sout, c32 ? 32 : 16, true, true, per_warp};
+    unsigned long long steps = 0;
+    deal_cones<kSvoWarps, true>(D, SvoDiffuseMarch{&S, &P.d, coef, sf, s_level, levels}, SvoFinish{D}, steps, ticket);
+    add_steps(step_counter, steps);
+}
+
+// One lane per specular cone of the aperture-grouped list, 32 at a time to
+// the warps as they free up.
+__global__ void __launch_bounds__(128) k_svo_specular(const __grid_constant__ TraceParams P,
+                                                      const __grid_constant__ SvoScene S,
+                                                      const vct_surface_sample* __restrict__ samples,
+                                                      const uint32_t* __restrict__ list,
+                                                      const unsigned int* __restrict__ spec_count,
+                                                      float* __restrict__ sout,
+                                                      unsigned long long* __restrict__ step_counter,
+                                                      unsigned int* __restrict__ ticket) {
+    const vct_cone_tracing_desc& d = P.d;
+    const uint32_t m = *spec_count;
+    const int lane = threadIdx.x & 31;
+    unsigned long long steps = 0;
+    for (;;) {
+        uint32_t c0 = 0;
+        if (lane == 0) c0 = atomicAdd(ticket, 32u);
+        c0 = __shfl_sync(0xffffffffu, c0, 0);
+        if (c0 >= m) break;
+        const uint32_t c = c0 + (uint32_t)lane;
+        if (c >= m) continue;
+        const uint32_t idx = __ldg(list + c);
+        const GSample g = load_sample(samples + idx, P.eye);
+        const float min_level = calc_min_level(d, g.wp);
+        const float vs = d.voxel_size * exp2f(min_level);
+        const float3 start = g.wp + g.normal * (vs * d.trace_start_offset);
+        const float3 sdir = normalize3(reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal));
+        const float coef = 2.0f * tanf(fmaxf(g.roughness, kMinSpecularAperture) * 0.5f);
+        const float4 r = svo_trace_cone(S, d, start, sdir, coef, min_level, fmaxf(kMinTraceStepFactor, d.voxel_size),
+                                        nullptr, 0, steps);
+        const float isi = d.indirect_specular_intensity;
+        reinterpret_cast<float4*>(sout)[idx] = svo_specular_out(
+            d.rendering_mode,
+            f3(r.x * g.specular_color.x * isi, r.y * g.specular_color.y * isi, r.z * g.specular_color.z * isi));
+    }
+    add_steps(step_counter, steps);
 }
 
 }  // namespace vct
@@ -214,26 +330,50 @@ extern "C" int vct_svo_cone_trace(const vct_cone_tracing_desc* desc, const vct_c
     S.pool = reinterpret_cast<const uint2*>(pool);
     VCT_CHECK_ARG(node_count < (1LL << 31), "vct_svo_cone_trace: node count out of range");
     S.nodes = (uint32_t)node_count;
+    S.dim = dim;
+    S.top = 30 - __builtin_clz(dim);
+    float ext[3];
     for (int a = 0; a < 3; ++a) {
-        S.bmin[a] = bb_min[a];
-        S.bmax[a] = bb_max[a];
+        ext[a] = bb_max[a] - bb_min[a];
+        S.c[a] = (bb_min[a] + bb_max[a]) * 0.5f;
     }
-    // the samples walked in the coherent order (normal class, then Morton), as the clipmap trace does
+    S.ev = fmaxf(ext[0], fmaxf(ext[1], ext[2])) * 0.5f;
+    const double scale = 0.5 * (double)dim / (double)S.ev;
+    S.a = (float)scale;
+    S.ga = (float)(fabs(scale) * 0x1p-20);
+    for (int a = 0; a < 3; ++a) {
+        const double off = 0.5 * (double)dim - (double)S.c[a] * scale;
+        S.b[a] = (float)off;
+        S.g0[a] = (float)((fabs((double)S.c[a] * scale) + (double)dim) * 0x1p-20);
+    }
+    S.min_radius = desc->voxel_size * desc->volume_dimension * 0.5f;
+    S.inv_r2 = (float)(1.0 / ((double)S.min_radius * (double)S.min_radius));
+    if (!std::isnormal(S.inv_r2)) S.inv_r2 = 0.0f;  // the shader's expression everywhere
+    S.inv_uvs = 1.0f / desc->voxel_size;
+    int exponent = 0;
+    S.uvs_pow2 = frexpf(desc->voxel_size, &exponent) == 0.5f && exponent > -120 && exponent < 120;
+    // counts of 2^30 samples or more run in chunks (the orders are 32-bit)
     cudaStream_t st = as_stream(stream);
-    SampleOrder so;
-    rc = sample_coherent_order(samples, n, P.d, &so, st);
-    if (rc != VCT_OK) return rc;
-    int64_t blocks = (n + 127) / 128;
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    unsigned int* ticket = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&ticket, sizeof(unsigned int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(unsigned int), st);
-    if (e == cudaSuccess) {
-        k_svo_trace<<<(int)blocks, 128, 0, st>>>(P, S, samples, n, so.order, dout, sout, cone_steps, ticket);
-        e = cudaGetLastError();
+    constexpr int64_t kChunk = 1LL << 30;
+    for (int64_t off = 0; off < n; off += kChunk) {
+        const int64_t m = n - off < kChunk ? n - off : kChunk;
+        const vct_surface_sample* smp = samples + off;
+        ExactPlan plan;
+        rc = exact_plan(smp, m, P.d, &plan, st);
+        if (rc != VCT_OK) return rc;
+        const int per_warp = deal_samples_per_warp(m, 152 * kSvoWarpsPerSm);
+        const int64_t gd = (m + (int64_t)per_warp * kSvoWarps - 1) / ((int64_t)per_warp * kSvoWarps);
+        k_svo_diffuse<<<(int)(gd > 152 * 8 ? 152 * 8 : gd), 32 * kSvoWarps, 0, st>>>(
+            P, S, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, plan.spec_count + 2, per_warp);
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) {
+            const int64_t gs = (m + 127) / 128;
+            k_svo_specular<<<(int)(gs > 152 * 8 ? 152 * 8 : gs), 128, 0, st>>>(
+                P, S, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, plan.spec_count + 1);
+            e = cudaGetLastError();
+        }
+        exact_plan_free(&plan, st);
+        if (e != cudaSuccess) return cuda_fail(e, "octree cone trace");
     }
-    if (ticket) cudaFreeAsync(ticket, st);
-    if (so.block) cudaFreeAsync(so.block, st);
-    if (e != cudaSuccess) return cuda_fail(e, "k_svo_trace");
     return VCT_OK;
 }

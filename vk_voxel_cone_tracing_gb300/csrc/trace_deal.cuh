@@ -53,10 +53,12 @@ inline int deal_samples_per_warp(int64_t n, int64_t warps) {
 
 // The positions base .. base + per_warp - 1 of the order on the calling warp.
 // `march(start, dir, start_level, steps)` traces one diffuse cone from `start`
-// and returns traceCone's (rgb, 1 - occlusion).  WARPS = warps per block.
-template <int WARPS, class Marcher>
-__device__ __forceinline__ void deal_diffuse_warp(const DealArgs& A, const Marcher& march, int64_t base,
-                                                  unsigned long long& steps) {
+// and returns traceCone's (rgb, 1 - occlusion); `finish(g, min_level, sum, idx)`
+// ends sample idx on its owner lane, `sum` being (0, 0, 0, 1) plus the cones'
+// results times their cosines in cone order.  WARPS = warps per block.
+template <int WARPS, class Marcher, class Finish>
+__device__ __forceinline__ void deal_cones_warp(const DealArgs& A, const Marcher& march, const Finish& finish,
+                                                int64_t base, unsigned long long& steps) {
     __shared__ float4 s_start[WARPS][32];
     __shared__ float4 s_norm[WARPS][32];
     __shared__ int s_cincl[WARPS][32];     // inclusive prefix of the pairs per cone
@@ -148,30 +150,45 @@ __device__ __forceinline__ void deal_diffuse_warp(const DealArgs& A, const March
             }
             __syncwarp();
         }
-        if (valid) {
-            const float inv_n = 1.0f / (float)A.ncones;
-            float4 ind = make_float4(acc.x * inv_n, acc.y * inv_n, acc.z * inv_n, acc.w * inv_n);
-            ind.w = ind.w * d.ambient_occlusion_factor;
-            ind.x = ind.x * (g.diffuse_color.x * d.indirect_diffuse_intensity);
-            ind.y = ind.y * (g.diffuse_color.y * d.indirect_diffuse_intensity);
-            ind.z = ind.z * (g.diffuse_color.z * d.indirect_diffuse_intensity);
-            const float3 direct = direct_term(P, g);
-            const bool spec = A.need_specular && has_specular_cone(g);
-            float4 dd[2];
-            write_outputs(P, g, min_level, ind, f3(0.f, 0.f, 0.f), direct, reinterpret_cast<float*>(&dd[0]),
-                          reinterpret_cast<float*>(&dd[1]));
-            reinterpret_cast<float4*>(A.dout)[idx] = dd[0];
-            if (!spec) reinterpret_cast<float4*>(A.sout)[idx] = dd[1];
-        }
+        if (valid) finish(g, min_level, acc, idx);
     }
+}
+
+// The end of a clipmap sample: normalisation, AO, albedo, direct term, the
+// rendering-mode switch and its stores.
+struct ClipmapFinish {
+    const DealArgs& A;
+    __device__ __forceinline__ void operator()(const GSample& g, float min_level, float4 acc, uint32_t idx) const {
+        const TraceParams& P = *A.P;
+        const vct_cone_tracing_desc& d = P.d;
+        const float inv_n = 1.0f / (float)A.ncones;
+        float4 ind = make_float4(acc.x * inv_n, acc.y * inv_n, acc.z * inv_n, acc.w * inv_n);
+        ind.w = ind.w * d.ambient_occlusion_factor;
+        ind.x = ind.x * (g.diffuse_color.x * d.indirect_diffuse_intensity);
+        ind.y = ind.y * (g.diffuse_color.y * d.indirect_diffuse_intensity);
+        ind.z = ind.z * (g.diffuse_color.z * d.indirect_diffuse_intensity);
+        const float3 direct = direct_term(P, g);
+        const bool spec = A.need_specular && has_specular_cone(g);
+        float4 dd[2];
+        write_outputs(P, g, min_level, ind, f3(0.f, 0.f, 0.f), direct, reinterpret_cast<float*>(&dd[0]),
+                      reinterpret_cast<float*>(&dd[1]));
+        reinterpret_cast<float4*>(A.dout)[idx] = dd[0];
+        if (!spec) reinterpret_cast<float4*>(A.sout)[idx] = dd[1];
+    }
+};
+
+template <int WARPS, class Marcher>
+__device__ __forceinline__ void deal_diffuse_warp(const DealArgs& A, const Marcher& march, int64_t base,
+                                                  unsigned long long& steps) {
+    deal_cones_warp<WARPS>(A, march, ClipmapFinish{A}, base, steps);
 }
 
 // Every warp of the grid over the order, per_warp positions at a time: with
 // TICKET (`ticket` zeroed before the launch), the items go to the warps as
 // they free up; without, by a static grid stride.
-template <int WARPS, bool TICKET = false, class Marcher>
-__device__ __forceinline__ void deal_diffuse(const DealArgs& A, const Marcher& march, unsigned long long& steps,
-                                             unsigned int* ticket = nullptr) {
+template <int WARPS, bool TICKET, class Marcher, class Finish>
+__device__ __forceinline__ void deal_cones(const DealArgs& A, const Marcher& march, const Finish& finish,
+                                           unsigned long long& steps, unsigned int* ticket) {
     if constexpr (TICKET) {
         const int lane = threadIdx.x & 31;
         for (;;) {
@@ -180,14 +197,20 @@ __device__ __forceinline__ void deal_diffuse(const DealArgs& A, const Marcher& m
             it = __shfl_sync(0xffffffffu, it, 0);
             const int64_t base = (int64_t)it * A.per_warp;
             if (base >= A.n) break;
-            deal_diffuse_warp<WARPS>(A, march, base, steps);
+            deal_cones_warp<WARPS>(A, march, finish, base, steps);
         }
         return;
     }
     const int64_t nwarps = (int64_t)gridDim.x * WARPS;
     for (int64_t base = ((int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5)) * A.per_warp; base < A.n;
          base += nwarps * A.per_warp)
-        deal_diffuse_warp<WARPS>(A, march, base, steps);
+        deal_cones_warp<WARPS>(A, march, finish, base, steps);
+}
+
+template <int WARPS, bool TICKET = false, class Marcher>
+__device__ __forceinline__ void deal_diffuse(const DealArgs& A, const Marcher& march, unsigned long long& steps,
+                                             unsigned int* ticket = nullptr) {
+    deal_cones<WARPS, TICKET>(A, march, ClipmapFinish{A}, steps, ticket);
 }
 
 // Adds a warp's step count to the counter (one atomic per warp).
