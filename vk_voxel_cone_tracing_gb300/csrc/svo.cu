@@ -12,7 +12,12 @@
 // within a depth is path order, and the distinct prefixes of the sorted paths
 // are the pool's nodes.  Consecutive fragments mostly share their leaf (the
 // samples of a pixel), so the sort runs over runs of them, and the fold reads
-// each run's fragments where they lie.
+// each run's fragments where they lie.  What bounds it is the one pass over
+// the fragments that finds the runs and the fold's chain.  Against a flag pass
+// over the fragments per level and a sort of every fragment by its leaf:
+// 58.4 M fragments at L = 9, fragments + build + trace 11.04 -> 7.13 ms (two
+// host readbacks in the build instead of eight); the room at L = 7, 2.01 ->
+// 1.43 ms.
 // Mips (octreeNodeMipmapWrite.comp) are computed per node: the shader
 // writes, for each power-of-two target level t <= 2^(L-1), the flagged nodes
 // at resolution t; a per-node pass over those windows gives the same values
