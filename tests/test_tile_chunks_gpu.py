@@ -1,0 +1,50 @@
+"""The coverage kernels' chunks take tiles from all over the list by its length (fewer than 2^18 tiles, 2^20, more):
+opacity, the deterministic injection and the octree's fragment list stay equal to the oracle's (or, for the longest
+list, to the same triangles rasterised in two halves)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LIGHT_DIR = (0.3, -1.0, 0.2)
+
+
+@pytest.mark.parametrize("R,n_random", [(16, 0), (64, 3), (64, 9000), (256, 2500)])
+def test_opacity_and_injection_equal_the_oracle(cuda, oracle, R, n_random):
+    torch = cuda
+    from vk_voxel_cone_tracing_gb300 import capi, clipmap, passes
+    from vk_voxel_cone_tracing_gb300.scene import room_scene
+    scene = room_scene(seed=8, n_random=n_random)
+    ds, ws = passes.DeviceScene(scene), passes.Workspace()
+    regions = clipmap.clip_regions((0.3, 2.5, -0.4), R)
+    rn = clipmap.regions_to_numpy(regions)
+    mask = 0x3F if R < 256 else 0x24
+    want = oracle.voxelize_opacity(scene, R, rn, level_mask=mask)
+    atlas = clipmap.new_atlas(R)
+    passes.voxelize_opacity(ds, regions, R, atlas, ws, level_mask=mask)
+    assert np.array_equal(atlas.cpu().numpy().view(np.uint32), want)
+    atlas.zero_()
+    passes.inject_radiance(ds, regions, R, None, passes.light_desc(LIGHT_DIR), capi.DirectionalLightShadowDesc(), atlas,
+                           ws, level_mask=mask)
+    want = oracle.inject_radiance(scene, R, rn, None, bytes(capi.DirectionalLightShadowDesc()), level_mask=mask)
+    assert np.array_equal(atlas.cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("triangles", [1, 20, 90000, 700000, 1300000])
+def test_fragment_list_is_its_halves(cuda, triangles):
+    """The list of a scene is the list of its first triangles followed by that of the rest."""
+    torch = cuda
+    import copy
+    from vk_voxel_cone_tracing_gb300 import capi, passes
+    from vk_voxel_cone_tracing_gb300.scene import terrain_scene
+    scene = terrain_scene(seed=5, target=max(triangles, 40), boxes=triangles // 300)
+    T, ws, sd = scene.indices.shape[0], passes.Workspace(), capi.DirectionalLightShadowDesc()
+    whole = passes.DeviceScene(scene)
+    lists = []
+    for lo, hi in ((0, T), (0, T // 3), (T // 3, T)):
+        part = copy.copy(scene)
+        part.indices, part.tri_material = scene.indices[lo:hi], scene.tri_material[lo:hi]
+        if hi > lo:
+            lists.append(passes.svo_fragments(passes.DeviceScene(part), 8, None, passes.light_desc(LIGHT_DIR), sd, ws,
+                                              bb_min=whole.bb_min, bb_max=whole.bb_max))
+    assert torch.equal(lists[0], torch.cat(lists[1:]))

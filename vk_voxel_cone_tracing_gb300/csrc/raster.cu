@@ -696,6 +696,7 @@ struct TilePlan {
     const uint32_t* tile_item;  // item of every tile
     uint32_t total;             // tiles
     unsigned int* ticket;       // the next chunk of 32 tiles a coverage warp takes (zeroed per launch)
+    int group;                  // of the launch: chunk_group
 };
 
 // Item of every tile: item i owns tiles [tile_end[i-1], tile_end[i]).  A warp
@@ -962,8 +963,31 @@ __device__ __forceinline__ uint32_t next_chunk(unsigned int* ticket, int lane) {
     return __shfl_sync(0xffffffffu, c, 0);
 }
 
-// Coverage kernels.  A warp takes 32 consecutive 8x8 tiles of (triangle,
-// level) items -- one per lane -- sets each up once into shared memory, then
+// The tile that lane `lane` of chunk `ch` takes: groups of 2^group
+// consecutive tiles, a chunk's groups a fixed stride apart.
+__device__ __forceinline__ uint32_t chunk_tile(uint32_t ch, uint32_t nchunks, int lane, int group) {
+    const uint32_t l = (uint32_t)lane;
+    return (((l >> group) * nchunks + ch) << group) + (l & ((1u << group) - 1u));
+}
+
+// log2 of the consecutive tiles a chunk takes together.  The 8-sample passes
+// spend up to 512 rounds on a chunk of 32 full tiles (a floor quad has
+// hundreds in a row) and a few on a chunk of small triangles, and the longest
+// chunk was the kernel's time: 85 % of the SM cycles idle on a 34k-triangle
+// room.  Chunks whose tiles come from all over the list are alike; many tiles
+// need less of it, and consecutive ones share their loads.  Measured (us at 32
+// / 8 / 4 / 2 consecutive): opacity + count of 206k tiles 322 / - / 92 / 68,
+// emission 209 / - / 62 / 44; octree count of 4.3M tiles 1202 / - / 1115 /
+// 1142; opacity + count of 5.6M tiles 1714 / - / 1755 / 1773.  The one-sample
+// passes (shadow, G-buffer) have cheap full tiles and keep 32: 114 against 122
+// / 127 us at 280k tiles.
+static int chunk_group(bool one_sample, uint32_t tiles) {
+    if (one_sample) return 5;
+    return tiles < (1u << 18) ? 0 : (tiles < (1u << 20) ? 1 : 3);
+}
+
+// Coverage kernels.  A warp takes 32 8x8 tiles of (triangle, level) items
+// (chunk_tile) -- one per lane -- sets each up once into shared memory, then
 // flattens the (tile, pixel) pairs of all 32 tiles and walks them 32 at a
 // time, one pixel (all of its samples) per lane, so every lane does the same
 // work however unequal the tiles are.  Pixel q of the flattened list belongs
@@ -994,7 +1018,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
     // chunks are dealt to the warps as they free up (a ticket), so unequal chunks do not leave SMs idle at the
     // end; every chunk's results depend only on its index
     for (uint32_t ch = next_chunk(plan.ticket, lane); ch < nchunks; ch = next_chunk(plan.ticket, lane)) {
-        const uint32_t g = ch * 32u + lane;
+        const uint32_t g = chunk_tile(ch, nchunks, lane, plan.group);
         uint32_t npx = 0;
         // the emit phase skips tiles whose count pass found no covered sample
         if (g < total && !(PHASE == P_WRITE && counts[g] == 0u)) {
@@ -1262,9 +1286,10 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
 }
 
 template <int KIND, int PHASE>
-static void launch_cover(const RasterArgs& A, const TilePlan& plan, uint32_t* counts, const unsigned long long* offs,
+static void launch_cover(const RasterArgs& A, TilePlan plan, uint32_t* counts, const unsigned long long* offs,
                          FragDesc* frags, int* err, cudaStream_t st) {
     const uint32_t nchunks = (plan.total + 31u) >> 5;
+    plan.group = chunk_group(KIND == K_SHADOW || KIND == K_GBUFFER, plan.total);
     int blocks = (int)((nchunks + 3u) >> 2);
     blocks = blocks < 1 ? 1 : (blocks > 152 * 16 ? 152 * 16 : blocks);
     // (an error of the zeroing is the thread's last error, which the callers' launch check reads)
@@ -1892,6 +1917,7 @@ static int plan_tiles(RasterArgs& A, vct_workspace_s* ws, size_t& off, TilePlan*
     plan->tile_item = tile_item;
     plan->total = total;
     plan->ticket = ticket;
+    plan->group = 0;
     return VCT_OK;
 }
 
