@@ -31,7 +31,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 # inlined into the single and the batched kernels, and with multiply-add contraction left to the compiler the
 # two could round a sample's diffuse sum differently (by one unit in the last place) from the same inputs.
 NO_FMA = {"clipmap_passes.cu", "trace_exact.cu", "raster.cu", "svo.cu", "svo_trace.cu", "composite.cu", "trace_grad.cu",
-          "trace_fast.cu"}
+          "trace_fast.cu", "frame_tail.cu"}
 
 
 def nvcc() -> str:

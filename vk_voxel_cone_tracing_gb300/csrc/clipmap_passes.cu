@@ -32,16 +32,6 @@ __global__ void k_clear_region(uint32_t* __restrict__ atlas, AtlasDims A, int3 r
 // Thread per texel position (cube_texel order: coalesced 4-byte RMW), all
 // faces; R is a power of two, so the (x, y, z) split is shifts.
 // `mirror` (0 = none): a texture array's surface that receives the same texels.
-// `touched` (may be null): texels whose bit is clear read as zero rgb.
-// (Both words are loaded unconditionally and selected, so the loads of a
-// thread's texels stay independent and in flight together.)
-__device__ __forceinline__ uint32_t rgb_of(const uint32_t* __restrict__ atlas, const uint32_t* __restrict__ touched,
-                                           int64_t i) {
-    const uint32_t r = atlas[i];
-    const uint32_t w = touched ? __ldg(touched + (i >> 5)) : 0xffffffffu;
-    return ((w >> (i & 31)) & 1u) ? (r & 0x00ffffffu) : 0u;
-}
-
 // Texel order of the passes that also store into a texture: a warp takes 16
 // x-neighbours of two neighbouring rows, so each 32-byte sector of the
 // array's block-linear layout (16 B of two neighbouring rows) is written
@@ -60,19 +50,13 @@ __device__ __forceinline__ void cube_texel(uint32_t t, int lg, int& x, int& y, i
     z = (int)(t >> (2 * lg));
 }
 
-// The alpha byte of opacity texel i in the alpha position of an RGBA8 word:
-// the reference's RGBA8 opacity atlas (OT = uint32_t) or the one-byte-per-
-// texel form (OT = uint8_t, the same texel order), which holds the alpha only.
+// Opacity texel i's alpha byte in place.
 __device__ __forceinline__ uint32_t opa_alpha(const uint32_t* __restrict__ opa, int64_t i) {
     return __ldg(opa + i) & 0xff000000u;
 }
-__device__ __forceinline__ uint32_t opa_alpha(const uint8_t* __restrict__ opa, int64_t i) {
-    return (uint32_t)__ldg(opa + i) << 24;
-}
 
-template <class OT>
-__global__ void k_copy_alpha(uint32_t* __restrict__ dst, const OT* __restrict__ src, AtlasDims A, int level,
-                             int lg, int faces, cudaSurfaceObject_t mirror, const uint32_t* __restrict__ touched) {
+__global__ void k_copy_alpha(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, AtlasDims A, int level,
+                             int lg, int faces, cudaSurfaceObject_t mirror) {
     const uint32_t n = 1u << (3 * lg);
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         int x, y, z;
@@ -85,7 +69,7 @@ __global__ void k_copy_alpha(uint32_t* __restrict__ dst, const OT* __restrict__ 
         uint32_t v[6];
 #pragma unroll
         for (int f = 0; f < 6; ++f)
-            if (f < faces) v[f] = rgb_of(dst, touched, i0 + A.rb * f) | opa_alpha(src, i0 + A.rb * f);
+            if (f < faces) v[f] = (dst[i0 + A.rb * f] & 0x00ffffffu) | opa_alpha(src, i0 + A.rb * f);
 #pragma unroll
         for (int f = 0; f < 6; ++f)
             if (f < faces) {
@@ -105,14 +89,9 @@ __device__ __forceinline__ uint4 opa_alpha4(const uint32_t* __restrict__ opa, in
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(opa + i));
     return make_uint4(v.x & 0xff000000u, v.y & 0xff000000u, v.z & 0xff000000u, v.w & 0xff000000u);
 }
-__device__ __forceinline__ uint4 opa_alpha4(const uint8_t* __restrict__ opa, int64_t i) {
-    const uint32_t b = __ldg(reinterpret_cast<const uint32_t*>(opa + i));
-    return make_uint4(b << 24, (b << 16) & 0xff000000u, (b << 8) & 0xff000000u, b & 0xff000000u);
-}
 
-template <class OT>
-__global__ void k_copy_alpha4(uint32_t* __restrict__ dst, const OT* __restrict__ src, AtlasDims A, int level,
-                              int faces, cudaSurfaceObject_t mirror, const uint32_t* __restrict__ touched) {
+__global__ void k_copy_alpha4(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, AtlasDims A, int level,
+                              int faces, cudaSurfaceObject_t mirror) {
     const int lane = threadIdx.x & 31;
     const uint32_t groups = (uint32_t)(A.rb * faces + 3) >> 2;  // x groups of a row
     const uint32_t g32 = (groups + 31u) & ~31u;                  // a row's groups padded to whole warps
@@ -130,14 +109,13 @@ __global__ void k_copy_alpha4(uint32_t* __restrict__ dst, const OT* __restrict__
         if (valid) {
             const uint4 d = *reinterpret_cast<const uint4*>(dst + i);
             const uint4 a = opa_alpha4(src, i);
-            const uint32_t w = touched ? __ldg(touched + (i >> 5)) : 0xffffffffu;
             v[0] = d.x, v[1] = d.y, v[2] = d.z, v[3] = d.w;
             const uint32_t av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int x = x0 + k, xf = x % A.rb;
                 if (x < A.rb * faces && xf >= 1 && xf <= A.R)
-                    v[k] = (((w >> ((i + k) & 31)) & 1u) ? (v[k] & 0x00ffffffu) : 0u) | av[k];
+                    v[k] = (v[k] & 0x00ffffffu) | av[k];
             }
             *reinterpret_cast<uint4*>(dst + i) = make_uint4(v[0], v[1], v[2], v[3]);
         }
@@ -390,13 +368,10 @@ __global__ void k_downsample_r8(uint8_t* __restrict__ atlas, const uint8_t* __re
 // restrict pointer: level l - 1 is not written by this pass).
 constexpr int kAlphaDsFacesPerRound = 2;
 
-template <class OT>
 __global__ void __launch_bounds__(128, 8) k_alpha_downsample(uint32_t* __restrict__ rad,
-                                                                    const uint32_t* __restrict__ prev,
-                                                                    const OT* __restrict__ opa, AtlasDims A,
-                                                                    int3 pmin, int level, int band, int lg,
-                                                                    cudaSurfaceObject_t mirror,
-                                                                    const uint32_t* __restrict__ touched) {
+                                                             const uint32_t* __restrict__ prev,
+                                                             const uint32_t* __restrict__ opa, AtlasDims A, int3 pmin,
+                                                             int level, int band, int lg, cudaSurfaceObject_t mirror) {
     const int half = A.R >> 1;
     const int pm[3] = {pmin.x, pmin.y, pmin.z};
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -413,7 +388,7 @@ __global__ void __launch_bounds__(128, 8) k_alpha_downsample(uint32_t* __restric
         uint32_t own6[6];
 #pragma unroll
         for (int f = 0; f < 6; ++f)
-            own6[f] = rgb_of(rad, touched, w0 + A.rb * f) | opa_alpha(opa, w0 + A.rb * f);
+            own6[f] = (rad[w0 + A.rb * f] & 0x00ffffffu) | opa_alpha(opa, w0 + A.rb * f);
         const int my = w[1] + 1 + A.rb * level, mz = w[2] + 1;
 #pragma unroll
         for (int f = 0; f < 6; ++f) {
@@ -453,7 +428,7 @@ __global__ void __launch_bounds__(128, 8) k_alpha_downsample(uint32_t* __restric
         uint32_t own6[6];
 #pragma unroll
         for (int f = 0; f < 6; ++f)
-            own6[f] = rgb_of(rad, touched, w0 + A.rb * f) | opa_alpha(opa, w0 + A.rb * f);
+            own6[f] = (rad[w0 + A.rb * f] & 0x00ffffffu) | opa_alpha(opa, w0 + A.rb * f);
         const int64_t c0 = A.index(ps[0], ps[1], ps[2]);
         const int64_t dy = A.W, dz = (int64_t)A.W * A.H;
 #pragma unroll
@@ -527,8 +502,8 @@ extern "C" int vct_clear_region(uint32_t* atlas, const vct_image_cleaning_desc* 
 
 namespace vct {
 
-int copy_alpha_pass(uint32_t* dst, const void* src, const vct_copy_alpha_desc* d, cudaSurfaceObject_t mirror,
-                    const uint32_t* touched, cudaStream_t st, bool src_r8) {
+int copy_alpha_pass(uint32_t* dst, const uint32_t* src, const vct_copy_alpha_desc* d, cudaSurfaceObject_t mirror,
+                    cudaStream_t st) {
     VCT_CHECK_ARG(dst && src && d, "vct_copy_alpha: null argument");
     VCT_CHECK_ARG(valid_resolution(d->clipmap_resolution), "vct_copy_alpha: resolution must be a power of two in [8,1024]");
     VCT_CHECK_ARG(d->clip_level >= 0 && d->clip_level < VCT_CLIP_LEVEL_COUNT, "vct_copy_alpha: clip level out of range");
@@ -539,30 +514,21 @@ int copy_alpha_pass(uint32_t* dst, const void* src, const vct_copy_alpha_desc* d
     const int lg = 31 - __builtin_clz((unsigned)A.R);
     const int64_t n = (int64_t)A.R * A.R * A.R;
     const int grid = grid_for(n, 256);
-    const bool aligned = (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;  // 16-byte row groups (R8: 4 bytes)
+    const bool aligned = (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;  // 16-byte row groups
     if (aligned) {
         const int64_t n4 = (int64_t)((((A.rb * d->face_count + 3) >> 2) + 31) & ~31) * A.R * A.R;
-        const int grid4 = grid_for(n4, 256);
-        if (src_r8)
-            k_copy_alpha4<<<grid4, 256, 0, st>>>(dst, static_cast<const uint8_t*>(src), A, d->clip_level,
-                                                 d->face_count, mirror, touched);
-        else
-            k_copy_alpha4<<<grid4, 256, 0, st>>>(dst, static_cast<const uint32_t*>(src), A, d->clip_level,
-                                                 d->face_count, mirror, touched);
-    } else if (src_r8)
-        k_copy_alpha<<<grid, 256, 0, st>>>(dst, static_cast<const uint8_t*>(src), A, d->clip_level, lg, d->face_count,
-                                           mirror, touched);
-    else
-        k_copy_alpha<<<grid, 256, 0, st>>>(dst, static_cast<const uint32_t*>(src), A, d->clip_level, lg, d->face_count,
-                                           mirror, touched);
+        k_copy_alpha4<<<grid_for(n4, 256), 256, 0, st>>>(dst, src, A, d->clip_level, d->face_count, mirror);
+    } else {
+        k_copy_alpha<<<grid, 256, 0, st>>>(dst, src, A, d->clip_level, lg, d->face_count, mirror);
+    }
     VCT_LAUNCH_CHECK();
     return VCT_OK;
 }
 
-int copy_alpha_downsample_pass(uint32_t* radiance, const void* opacity, const vct_downsample_desc* d,
-                               cudaSurfaceObject_t mirror, const uint32_t* touched, cudaStream_t st, bool opa_r8) {
+int copy_alpha_downsample_pass(uint32_t* radiance, const uint32_t* opacity, const vct_downsample_desc* d,
+                               cudaSurfaceObject_t mirror, cudaStream_t st) {
     VCT_CHECK_ARG(radiance && opacity && d, "vct_copy_alpha_downsample: null argument");
-    VCT_CHECK_ARG((const void*)radiance != opacity, "vct_copy_alpha_downsample: radiance and opacity atlases must differ");
+    VCT_CHECK_ARG(radiance != opacity, "vct_copy_alpha_downsample: radiance and opacity atlases must differ");
     VCT_CHECK_ARG(valid_resolution(d->clipmap_resolution),
                   "vct_copy_alpha_downsample: resolution must be a power of two in [8,1024]");
     VCT_CHECK_ARG(d->clip_level >= 1 && d->clip_level < VCT_CLIP_LEVEL_COUNT,
@@ -575,12 +541,7 @@ int copy_alpha_downsample_pass(uint32_t* radiance, const void* opacity, const vc
     const int lg = 31 - __builtin_clz((unsigned)A.R);
     const int grid = grid_for(n, 128);
     const int band = d->downsample_region_size, l = d->clip_level;
-    if (opa_r8)
-        k_alpha_downsample<<<grid, 128, 0, st>>>(radiance, radiance, static_cast<const uint8_t*>(opacity), A, pm, l,
-                                                 band, lg, mirror, touched);
-    else
-        k_alpha_downsample<<<grid, 128, 0, st>>>(radiance, radiance, static_cast<const uint32_t*>(opacity), A, pm, l,
-                                                 band, lg, mirror, touched);
+    k_alpha_downsample<<<grid, 128, 0, st>>>(radiance, radiance, opacity, A, pm, l, band, lg, mirror);
     VCT_LAUNCH_CHECK();
     return VCT_OK;
 }
@@ -622,7 +583,7 @@ static int mirror_surface(vct_texture_s* t, int R, const char* who, cudaSurfaceO
 }  // namespace vct
 
 extern "C" int vct_copy_alpha(uint32_t* dst, const uint32_t* src, const vct_copy_alpha_desc* d, void* stream) {
-    return copy_alpha_pass(dst, src, d, 0, nullptr, as_stream(stream), false);
+    return copy_alpha_pass(dst, src, d, 0, as_stream(stream));
 }
 
 extern "C" int vct_copy_alpha_downsample(uint32_t* radiance, const uint32_t* opacity, const vct_downsample_desc* d,
@@ -632,7 +593,7 @@ extern "C" int vct_copy_alpha_downsample(uint32_t* radiance, const uint32_t* opa
     int rc = mirror_surface(mirror, d->clipmap_resolution,
                             "vct_copy_alpha_downsample: the mirror must be an RGBA8 texture of the same resolution", &surf);
     if (rc != VCT_OK) return rc;
-    return copy_alpha_downsample_pass(radiance, opacity, d, surf, nullptr, as_stream(stream), false);
+    return copy_alpha_downsample_pass(radiance, opacity, d, surf, as_stream(stream));
 }
 
 extern "C" int vct_wrap_border(uint32_t* atlas, const vct_border_wrapping_desc* d, void* stream) {

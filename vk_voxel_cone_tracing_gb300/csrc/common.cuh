@@ -10,11 +10,11 @@
 #include "../../include/vct_capi.h"
 
 // Device scratch arena of the raster / SVO passes (vct_workspace), a
-// second buffer that outlives a pass within one frame (the frame's
-// touched-texel bitmap), and a side stream with two events and a workspace
-// of its own, on which a frame runs the passes that are independent of the
-// main stream's work beside them (created on first use, on the device
-// current then).
+// second buffer that outlives a pass within one frame (the frame's voxel
+// bitmaps), and two side streams with two events each (and a workspace for the
+// first), on which a frame runs the passes that are independent of the main
+// stream's work beside them (created on first use, on the device current
+// then).
 struct vct_workspace_s {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -22,6 +22,8 @@ struct vct_workspace_s {
     size_t aux_bytes = 0;
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t side2 = nullptr;
+    cudaEvent_t fork2 = nullptr, join2 = nullptr;
     int side_device = -1;
     vct_workspace_s* side_ws = nullptr;  // the scratch of the passes run on the side stream
 };
@@ -42,32 +44,46 @@ int texture_format(const vct_texture_s* t);
 // Copy-alpha of one level, and copy-alpha + radiance mip of one level >= 1,
 // optionally mirroring every texel they write into a texture array's surface
 // (clipmap_passes.cu).
-// `touched` (may be null): a bitmap over the atlas's texel indices; a texel
-// whose bit is clear is read as zero rgb (the frame's radiance clear folded
-// into these passes).
-// `opa_r8`: the opacity atlas is the one-byte-per-texel form (alpha only).
-int copy_alpha_pass(uint32_t* dst, const void* src, const vct_copy_alpha_desc* d, cudaSurfaceObject_t mirror,
-                    const uint32_t* touched, cudaStream_t st, bool src_r8);
-int copy_alpha_downsample_pass(uint32_t* radiance, const void* opacity, const vct_downsample_desc* d,
-                               cudaSurfaceObject_t mirror, const uint32_t* touched, cudaStream_t st, bool opa_r8);
+int copy_alpha_pass(uint32_t* dst, const uint32_t* src, const vct_copy_alpha_desc* d, cudaSurfaceObject_t mirror,
+                    cudaStream_t st);
+int copy_alpha_downsample_pass(uint32_t* radiance, const uint32_t* opacity, const vct_downsample_desc* d,
+                               cudaSurfaceObject_t mirror, cudaStream_t st);
+
+// A deterministic frame's voxel bitmaps, bit ((level R + z) R + y) R + x of the
+// levels' R^3 voxels (frame_bitmap_bytes each): voxels the opacity pass marked
+// (full revoxelisation; null in a toroidal update), voxels the injection lit
+// (all six faces of their radiance texels are written), and mip targets with a
+// nonzero face.  The streaming passes over them are in frame_tail.cu.
+struct FrameBits {
+    uint32_t *lit, *opaque, *nonzero;
+};
+size_t frame_bitmap_bytes(int R);
+// The opacity atlas (RGBA8, or one byte per texel) from `opaque`, borders zero.
+int frame_opacity_fill(void* atlas, bool r8, int R, const uint32_t* opaque, cudaStream_t st);
+// The due levels' copy-alpha (`opacity` is read only without B.opaque), and the
+// mips of the due levels 1..5.
+int frame_radiance_fill(uint32_t* radiance, const uint32_t* opacity, const FrameBits& B, int R, uint32_t due,
+                        cudaSurfaceObject_t mirror, cudaStream_t st);
+int frame_radiance_mips(uint32_t* radiance, const void* opacity, bool r8, const FrameBits& B,
+                        const vct_clipmap_region regions[6], int R, uint32_t due, cudaSurfaceObject_t mirror,
+                        cudaStream_t st);
 // The one-byte opacity form's mips 1..5 and border wrap (clipmap_passes.cu).
 int opacity_r8_mips(uint8_t* atlas, const vct_clipmap_region regions[6], int R, cudaStream_t st);
 int wrap_border_r8(uint8_t* atlas, int R, cudaStream_t st);
 
-// The frame's rasterised passes with the deterministic injection, up to the
-// fold (raster.cu): opacity clear + voxelisation + mips + border, shadow
-// depth, clear of the due radiance levels and the injection.
+// A frame's passes with the deterministic injection (raster.cu): opacity
+// voxelisation, mips and border, shadow depth, injection, and the due radiance
+// levels' copy-alpha and mips, mirrored into `mirror` (0: none).
 // The radiance levels due are not cleared: the fold starts their texels from
-// zero and marks each texel it writes in *touched (a bitmap over the atlas's
-// texel indices, in the workspace's second buffer), and the copy-alpha / mip
-// passes read unmarked texels as zero rgb -- the cleared result.
+// zero, stores all faces of each voxel it lights and marks it in *bits, and the
+// passes after it take unmarked voxels as zero rgb -- the cleared result.
 // With nslabs >= 0 the opacity atlas is updated toroidally: only the listed
 // slabs are cleared and revoxelised (levels with a whole-region slab in
 // full), and only the revoxelised levels' opacity mips are rebuilt.
 int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const vct_clipmap_region regions[6],
                         uint32_t due, const vct_clipmap_region* slabs, const int32_t* slab_levels, int nslabs,
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
-                        const uint32_t** touched, cudaStream_t st);
+                        cudaSurfaceObject_t mirror, FrameBits* bits, cudaStream_t st);
 
 // ---------------------------------------------------------------- errors
 void set_error(const std::string& msg);

@@ -353,7 +353,7 @@ struct RasterArgs {
     // p.a <= slab_hi[l][a]; an empty interval has lo > hi)
     uint32_t slab_levels;
     float slab_lo[6][3], slab_hi[6][3];
-    int opa_r8;  // the opacity atlas holds one byte per texel (alpha only)
+    uint32_t* opa_bits;  // the opacity pass marks its voxels here, one bit each (see FrameBits), instead of in the atlas
 };
 
 // A fragment at world position p of a slab-restricted level is kept when it
@@ -547,6 +547,15 @@ __device__ inline int3 clip_image_coords(const vct_voxelization_desc& d, float3 
         ic[a] = ((int)(f * (float)R)) & (R - 1);  // f >= 0 and R a power of two: the value % R
     }
     return make_int3(ic[0] + 1, ic[1] + 1 + (R + 2) * (int)d.clip_level, ic[2] + 1);
+}
+
+// Sets the bit of the voxel at image coordinates ic (clip_image_coords) of a
+// level: samples share voxels, so most find it set already (a stale clear bit
+// costs an atomic, a set one never clears).
+__device__ __forceinline__ void mark_voxel(uint32_t* __restrict__ bits, int R, int lvl, int3 ic) {
+    const int64_t i = (((int64_t)lvl * R + (ic.z - 1)) * R + (ic.y - 1 - (R + 2) * lvl)) * R + (ic.x - 1);
+    const uint32_t m = 1u << (i & 31);
+    if (!(bits[i >> 5] & m)) atomicOr(bits + (i >> 5), m);
 }
 
 __device__ inline uint32_t conv_rgba8(float x, float y, float z, float w) {
@@ -1162,12 +1171,9 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                             const int3 ic = clip_image_coords(d, wp);
                             if (ic.x == last_ic.x && ic.y == last_ic.y && ic.z == last_ic.z) continue;
                             last_ic = ic;
-                            if (A.opa_r8) {
-                                uint8_t* a8 = reinterpret_cast<uint8_t*>(A.atlas);
-                                for (int f = 0; f < 6; ++f) a8[AD.index(ic.x + (A.R + 2) * f, ic.y, ic.z)] = 0xFFu;
-                            } else {
+                            if (A.opa_bits) mark_voxel(A.opa_bits, A.R, lvl, ic);
+                            else
                                 for (int f = 0; f < 6; ++f) A.atlas[AD.index(ic.x + (A.R + 2) * f, ic.y, ic.z)] = 0xFFFFFFFFu;
-                            }
                         } else if (KIND == K_INJECT) {
                             const vct_gltf_shade_material mat = material_of(A.s, T.meta >> 3);
                             const float3 wp = interp3(b, T.p);
@@ -1213,11 +1219,10 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                               qy = __shfl_up_sync(FULL, ic.y, 1), qz = __shfl_up_sync(FULL, ic.z, 1);
                     const bool dup = lane > 0 && po == o && qx == ic.x && qy == ic.y && qz == ic.z;
                     if (keep && !dup) {
-                        const AtlasDims AD(A.R);
-                        if (A.opa_r8) {
-                            uint8_t* a8 = reinterpret_cast<uint8_t*>(A.atlas);
-                            for (int f = 0; f < 6; ++f) a8[AD.index(ic.x + (A.R + 2) * f, ic.y, ic.z)] = 0xFFu;
+                        if (A.opa_bits) {
+                            mark_voxel(A.opa_bits, A.R, (int)(S[jo].meta & 7u), ic);
                         } else {
+                            const AtlasDims AD(A.R);
                             for (int f = 0; f < 6; ++f) A.atlas[AD.index(ic.x + (A.R + 2) * f, ic.y, ic.z)] = 0xFFFFFFFFu;
                         }
                     }
@@ -1548,7 +1553,8 @@ struct FoldArgs {
     const uint32_t* heads;
     const uint32_t* nheads;
     uint32_t* atlas;
-    uint32_t* touched;  // the frame's path (else null): texels start from zero, each one written is marked in this bitmap
+    uint32_t* lit;  // the frame's path (else null): texels start from zero, all six faces of a listed voxel are stored
+                    // and its bit (at its key) is set in this bitmap
     uint32_t* long_list;
     uint32_t* nlong;
     int R;
@@ -1562,10 +1568,9 @@ __device__ __forceinline__ int64_t voxel_texel(Key key, int R) {
     return AtlasDims(R).index(x + 1, y + 1 + (R + 2) * l, z + 1);
 }
 
-__device__ __forceinline__ void store_cell(uint32_t* __restrict__ atlas, uint32_t* __restrict__ touched, int64_t i,
-                                           uint32_t cell) {
-    atlas[i] = cell;
-    if (touched) atomicOr(touched + (i >> 5), 1u << (i & 31));
+template <class Key>
+__device__ __forceinline__ void mark_lit(uint32_t* __restrict__ lit, Key key) {
+    atomicOr(lit + (key >> 5), 1u << ((uint32_t)key & 31u));
 }
 
 // Whether a sample with these flags adds to face f.
@@ -1611,10 +1616,12 @@ __global__ void __launch_bounds__(128) k_inject_fold(const FoldArgs<Key, Run> F)
         const uint32_t v = v0 + (threadIdx.x & 31u) / G;
         uint32_t h = 0u, h1 = 0u;
         int64_t texel = 0;  // of the axis's even face
+        Key key = 0;
         if (v < voxels) {
             h = F.heads[v];
             h1 = F.heads[v + 1];
-            texel = voxel_texel(F.keys[h], F.R) + (F.R + 2) * (int64_t)(2 * axis);
+            key = F.keys[h];
+            texel = voxel_texel(key, F.R) + (F.R + 2) * (int64_t)(2 * axis);
         }
         bool is_long = h1 - h > kLongVoxelRuns;
         if (__any_sync(FULL, h1 - h > kLongVoxelSamples / 32u && !is_long)) {
@@ -1626,12 +1633,13 @@ __global__ void __launch_bounds__(128) k_inject_fold(const FoldArgs<Key, Run> F)
             is_long = is_long || sum > kLongVoxelSamples;
         }
         if (is_long) h1 = h;
+        const bool mine = h < h1;  // a voxel of the warp's, not a long one
         AvgCell even = avg_cell(0u), odd = even;
-        if (!F.touched && h < h1) {
+        if (!F.lit && mine) {
             even = avg_cell(F.atlas[texel]);
             odd = avg_cell(F.atlas[texel + F.R + 2]);
         }
-        uint32_t written = 0u;
+        uint32_t written = F.lit && mine ? 3u : 0u;
         uint32_t t = 0u, total = 0u, incl = 0u, len = 0u, start = 0u;  // the fetched runs, and the next of their samples
         float4 c = make_float4(0.f, 0.f, 0.f, 0.f), w = c;
         unsigned have = 0u;  // lanes whose sample is lit
@@ -1645,9 +1653,9 @@ __global__ void __launch_bounds__(128) k_inject_fold(const FoldArgs<Key, Run> F)
             const bool refill = t >= total && h < h1;
             if (__any_sync(FULL, refill)) {
                 Run r = 0;
-                const bool mine = refill && h + (uint32_t)lg < h1;
-                if (mine) r = F.runs[h + (uint32_t)lg];
-                const uint32_t nl = mine ? (uint32_t)(r & 31u) + 1u : 0u;
+                const bool some = refill && h + (uint32_t)lg < h1;
+                if (some) r = F.runs[h + (uint32_t)lg];
+                const uint32_t nl = some ? (uint32_t)(r & 31u) + 1u : 0u;
                 uint32_t ni = nl;
 #pragma unroll
                 for (int o = 1; o < G; o <<= 1) {
@@ -1704,8 +1712,10 @@ __global__ void __launch_bounds__(128) k_inject_fold(const FoldArgs<Key, Run> F)
             if (!__any_sync(FULL, more)) break;
         }
         if (lg < 3) {
-            if (written & 1u) store_cell(F.atlas, F.touched, texel, avg_word(even));
-            if (written & 2u) store_cell(F.atlas, F.touched, texel + F.R + 2, avg_word(odd));
+            if (written & 1u) F.atlas[texel] = avg_word(even);
+            if (written & 2u) F.atlas[texel + F.R + 2] = avg_word(odd);
+        } else if (F.lit && mine) {
+            mark_lit(F.lit, key);
         }
     }
 }
@@ -1738,7 +1748,7 @@ __global__ void __launch_bounds__(kLongThreads) k_inject_fold_long(const FoldArg
         if ((h1 - h0 > kGiantVoxelRuns) != (kLongThreads == 1024)) continue;
         const int64_t base = voxel_texel(F.keys[h0], F.R);
         if (threadIdx.x < 6) {
-            const uint32_t c = F.touched ? 0u : F.atlas[base + (F.R + 2) * (int)threadIdx.x];
+            const uint32_t c = F.lit ? 0u : F.atlas[base + (F.R + 2) * (int)threadIdx.x];
             s_cell[threadIdx.x] = c;
             s_k0[threadIdx.x] = (256u - (c >> 24)) & 255u;
             s_count[threadIdx.x] = 0u;
@@ -1828,7 +1838,8 @@ __global__ void __launch_bounds__(kLongThreads) k_inject_fold_long(const FoldArg
                         avg_step(cell, inject_value(make_float3(c[u].x, c[u].y, c[u].z), wk[u],
                                                     __float_as_uint(c[u].w)));
             }
-            if (count) store_cell(F.atlas, F.touched, base + (F.R + 2) * (int)f, avg_word(cell));
+            if (count || F.lit) F.atlas[base + (F.R + 2) * (int)f] = avg_word(cell);
+            if (f == 0 && F.lit) mark_lit(F.lit, F.keys[h0]);
         }
         __syncthreads();  // the shared lists are rewritten by the next voxel
     }
@@ -2036,7 +2047,7 @@ static int inject_prepare(RasterArgs& C, RasterArgs& I, vct_workspace_s* ws, cud
 // it as one element.  The count of runs is read back for the sort (a frame
 // keeps the GPU busy meanwhile with its opacity mips on the side stream).
 template <class Key, class Run>
-static int inject_group_and_fold(const RasterArgs& I, const InjectState& S, uint32_t* touched, vct_workspace_s* ws,
+static int inject_group_and_fold(const RasterArgs& I, const InjectState& S, uint32_t* lit, vct_workspace_s* ws,
                                  cudaStream_t side, cudaStream_t st) {
     const uint32_t nfrag = S.nfrag, groups = (nfrag + 31u) >> 5;
     const size_t r4 = a256(4 * (size_t)nfrag + 4), k4 = sizeof(Key) == 8 ? 2 * r4 : r4;
@@ -2070,11 +2081,11 @@ static int inject_group_and_fold(const RasterArgs& I, const InjectState& S, uint
     tb = S.temp_bytes;
     VCT_CUDA_TRY(cub::DeviceSelect::If(tmp, tb, thrust::counting_iterator<uint32_t>(0u), heads, tally,
                                        (int64_t)runs + 1, VoxelHead<Key>{keys_a, runs}, st));
-    const FoldArgs<Key, Run> F{S.fr, keys_a, runs_b, heads, tally, I.atlas, touched, (uint32_t*)keys_b, tally + 1, I.R};
-    // the few long voxels beside the others, on the side stream where there is one
+    const FoldArgs<Key, Run> F{S.fr, keys_a, runs_b, heads, tally, I.atlas, lit, (uint32_t*)keys_b, tally + 1, I.R};
+    // the few long voxels beside the others, on a side stream where there is one
     if (side) {
-        VCT_CUDA_TRY(cudaEventRecord(ws->fork, st));
-        VCT_CUDA_TRY(cudaStreamWaitEvent(side, ws->fork, 0));
+        VCT_CUDA_TRY(cudaEventRecord(ws->fork2, st));
+        VCT_CUDA_TRY(cudaStreamWaitEvent(side, ws->fork2, 0));
     }
     cudaStream_t lst = side ? side : st;
     k_inject_long<Key, Run><<<grid_of(runs, 256), 256, 0, lst>>>(F);
@@ -2085,15 +2096,19 @@ static int inject_group_and_fold(const RasterArgs& I, const InjectState& S, uint
     VCT_LAUNCH_CHECK();
     k_inject_fold<Key, Run><<<grid_of((int64_t)runs * 4, 128, 152 * 64), 128, 0, st>>>(F);
     VCT_LAUNCH_CHECK();
+    if (side) {
+        VCT_CUDA_TRY(cudaEventRecord(ws->join2, side));
+        VCT_CUDA_TRY(cudaStreamWaitEvent(st, ws->join2, 0));
+    }
     return VCT_OK;
 }
 
-// `side` (may be null): the frame's side stream, joined to `st` by the caller.
-static int inject_finish(const RasterArgs& I, const InjectState& S, uint32_t* touched, vct_workspace_s* ws,
+// `side` (may be null): a stream of the workspace's for the long voxels, joined to `st` again.
+static int inject_finish(const RasterArgs& I, const InjectState& S, uint32_t* lit, vct_workspace_s* ws,
                          cudaStream_t side, cudaStream_t st) {
     if (S.nfrag == 0) return VCT_OK;
-    return S.wide ? inject_group_and_fold<unsigned long long, unsigned long long>(I, S, touched, ws, side, st)
-                  : inject_group_and_fold<uint32_t, uint32_t>(I, S, touched, ws, side, st);
+    return S.wide ? inject_group_and_fold<unsigned long long, unsigned long long>(I, S, lit, ws, side, st)
+                  : inject_group_and_fold<uint32_t, uint32_t>(I, S, lit, ws, side, st);
 }
 
 static void fill_clipmap_levels(RasterArgs& A, const vct_clipmap_region* regions, int R, uint32_t level_mask) {
@@ -2157,8 +2172,14 @@ extern "C" int vct_workspace_destroy(vct_workspace_s* w) {
         e2 = cudaStreamDestroy(w->side);
         if (e == cudaSuccess) e = e2;
     }
-    if (w->fork) cudaEventDestroy(w->fork);
-    if (w->join) cudaEventDestroy(w->join);
+    if (w->side2) {
+        cudaError_t e2 = cudaStreamSynchronize(w->side2);
+        if (e == cudaSuccess) e = e2;
+        e2 = cudaStreamDestroy(w->side2);
+        if (e == cudaSuccess) e = e2;
+    }
+    for (cudaEvent_t ev : {w->fork, w->join, w->fork2, w->join2})
+        if (ev) cudaEventDestroy(ev);
     if (w->side_ws) {
         const int rc = vct_workspace_destroy(w->side_ws);
         if (rc != VCT_OK && e == cudaSuccess) e = cudaErrorUnknown;
@@ -2655,15 +2676,15 @@ extern "C" int vct_gbuffer(const vct_scene* scene, const vct_cam_matrix* cam, in
 
 namespace vct {
 
-// The rasterised part of a frame with the deterministic injection
-// (Application::run's VoxelizationPass, RSMPass and RadianceInjectionPass up to
-// the fold).  The opacity voxelisation and the injection's coverage count
-// share one tile plan and one coverage pass -- their items (every triangle at
-// every level, the same projections and viewport) are the same -- so the
-// order is: clear opacity, shadow depth (it does not depend on the atlases),
-// opacity + count + emit, opacity mips, border, clear of the due radiance
-// levels, then shading, sort and fold.  The results equal the passes run one
-// by one in the reference's order.
+// A frame's passes with the deterministic injection (Application::run's
+// VoxelizationPass, RSMPass and RadianceInjectionPass).  The opacity
+// voxelisation and the injection's coverage count share one tile plan and one
+// coverage pass -- their items (every triangle at every level, the same
+// projections and viewport) are the same.  Beside each other run: the shadow
+// depth, and opacity + count + emission; the opacity atlas (written from the
+// voxel bits), its mips and border, and the shading, sort, fold and the
+// radiance outside the mips' blocks; then the radiance mips.  The results
+// equal the passes run one by one in the reference's order.
 // The workspace's side stream, created on first use on the current device
 // (non-blocking, with its fork and join events); null when the current
 // device is not the one it was created on (the frame then runs serially).
@@ -2680,9 +2701,24 @@ static cudaStream_t side_stream(vct_workspace_s* ws) {
         cudaStreamDestroy(s);
         return nullptr;
     }
+    cudaStream_t s2 = nullptr;
+    cudaEvent_t a2 = nullptr, b2 = nullptr;
+    if (cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&a2, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b2, cudaEventDisableTiming) != cudaSuccess) {
+        if (a2) cudaEventDestroy(a2);
+        if (s2) cudaStreamDestroy(s2);
+        cudaEventDestroy(a);
+        cudaEventDestroy(b);
+        cudaStreamDestroy(s);
+        return nullptr;
+    }
     ws->side = s;
     ws->fork = a;
     ws->join = b;
+    ws->side2 = s2;
+    ws->fork2 = a2;
+    ws->join2 = b2;
     ws->side_device = dev;
     ws->side_ws = new vct_workspace_s();
     return s;
@@ -2705,15 +2741,15 @@ static int join_side(vct_workspace_s* ws, cudaStream_t side, cudaStream_t st) {
 int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const vct_clipmap_region regions[6],
                         uint32_t due, const vct_clipmap_region* slabs, const int32_t* slab_levels, int nslabs,
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
-                        const uint32_t** touched_out, cudaStream_t st) {
+                        cudaSurfaceObject_t mirror, FrameBits* bits_out, cudaStream_t st) {
     const int R = f->clipmap_resolution;
     void* stream = st;
     int rc;
     const bool toroidal = nslabs >= 0;
     SlabPlan P;
     if (toroidal && (rc = slab_plan(regions, R, slabs, slab_levels, nslabs, &P)) != VCT_OK) return rc;
-    // the touched-texel bitmap, one bit per atlas texel, cleared every frame
-    const size_t bm_bytes = a256(((size_t)AtlasDims(R).texels() + 31) / 32 * 4);
+    // the voxel bitmaps, one bit per voxel of the six levels each, cleared every frame
+    const size_t map_bytes = frame_bitmap_bytes(R), bm_bytes = (toroidal ? 1 : 3) * map_bytes;
     if (ws->aux_bytes < bm_bytes) {
         if (ws->aux) {
             VCT_CUDA_TRY(cudaDeviceSynchronize());
@@ -2724,9 +2760,11 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
         VCT_CUDA_TRY(cudaMalloc(&ws->aux, bm_bytes));
         ws->aux_bytes = bm_bytes;
     }
-    uint32_t* touched = (uint32_t*)ws->aux;
-    VCT_CUDA_TRY(cudaMemsetAsync(touched, 0, bm_bytes, st));
-    *touched_out = touched;
+    FrameBits& B = *bits_out;
+    B.lit = (uint32_t*)ws->aux;
+    B.opaque = toroidal ? nullptr : (uint32_t*)((char*)ws->aux + map_bytes);
+    B.nonzero = toroidal ? nullptr : (uint32_t*)((char*)ws->aux + 2 * map_bytes);
+    VCT_CUDA_TRY(cudaMemsetAsync(ws->aux, 0, bm_bytes, st));
     // Two stretches run on the side stream (with its own workspace), beside
     // main-stream work they share no buffer with: the shadow pass beside the
     // opacity clear, voxelisation and injection count / emission (the shadow
@@ -2738,11 +2776,8 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
     vct_workspace_s* sws = side ? ws->side_ws : ws;
     if (side && (rc = fork_side(ws, side, st)) != VCT_OK) return rc;
     const bool r8 = f->opacity_format == VCT_OPACITY_R8;  // (full revoxelisation only: checked by the caller)
-    if (toroidal) rc = clear_slabs(opacity, R, slabs, slab_levels, nslabs, stream);
-    else if (r8) rc = cudaMemsetAsync(opacity, 0, (size_t)AtlasDims(R).texels(), st) == cudaSuccess
-                          ? VCT_OK : fail(VCT_E_CUDA, "cudaMemsetAsync (opacity clear)");
-    else rc = vct_clear_atlas(opacity, R, stream);
-    if (rc != VCT_OK) return rc;
+    // a full revoxelisation marks bits; the whole atlas is written from them below
+    if (toroidal && (rc = clear_slabs(opacity, R, slabs, slab_levels, nslabs, st)) != VCT_OK) return rc;
     vct_shadow_map sm = {nullptr, 0, 0};
     if (f->shadow_width > 0) {
         if ((rc = vct_shadow_depth(scene, &f->light_shadow, shadow_depth, f->shadow_width, f->shadow_height, sws,
@@ -2768,12 +2803,11 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
         if (toroidal) apply_slabs(C, P);
         C.items = scene->triangle_count * C.nlevels;
         C.atlas = opacity;
-        C.opa_r8 = r8 ? 1 : 0;
+        C.opa_bits = B.opaque;
         C.count_levels = due;
         I = C;  // the injection's args over the same items
         I.kind = K_INJECT;
         I.atlas = radiance;
-        I.opa_r8 = 0;
         if ((rc = fill_light(I, &sm, &f->light, &f->light_shadow)) != VCT_OK) return rc;
         for (;;) {
             rc = inject_prepare<K_OPA_COUNT>(C, I, ws, st, &S);
@@ -2784,6 +2818,7 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
     // the shading below reads the shadow map; the mips read the voxelised opacity
     if (side && (rc = join_side(ws, side, st)) != VCT_OK) return rc;
     if (side && (rc = fork_side(ws, side, st)) != VCT_OK) return rc;
+    if (!toroidal && (rc = frame_opacity_fill(opacity, r8, R, B.opaque, ost)) != VCT_OK) return rc;
     if (r8) {
         if ((rc = opacity_r8_mips(reinterpret_cast<uint8_t*>(opacity), regions, R, ost)) != VCT_OK) return rc;
     } else if (!toroidal) {
@@ -2805,11 +2840,16 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
     else rc = vct_wrap_border(opacity, &bw, ost);
     if (rc != VCT_OK) return rc;
     // the due radiance levels' clear is folded into the fold (texels start from
-    // zero) and the copy-alpha / mip passes (unmarked texels read as zero rgb)
-    if (scene->triangle_count > 0 && (rc = inject_finish(I, S, touched, ws, side, st)) != VCT_OK) return rc;
-    // the copy-alpha and radiance mip passes that follow read the final opacity
+    // zero) and the copy-alpha / mip passes (unmarked voxels read as zero rgb)
+    if (scene->triangle_count > 0 && (rc = inject_finish(I, S, B.lit, ws, side ? ws->side2 : nullptr, st)) != VCT_OK)
+        return rc;
+    // The radiance of the due levels takes its alpha from the voxel bits, beside
+    // the opacity mips; the radiance mips (and the toroidal update's alpha) read
+    // the final opacity.
+    if (!toroidal && (rc = frame_radiance_fill(radiance, nullptr, B, R, due, mirror, st)) != VCT_OK) return rc;
     if (side && (rc = join_side(ws, side, st)) != VCT_OK) return rc;
-    return VCT_OK;
+    if (toroidal && (rc = frame_radiance_fill(radiance, opacity, B, R, due, mirror, st)) != VCT_OK) return rc;
+    return frame_radiance_mips(radiance, opacity, r8, B, regions, R, due, mirror, st);
 }
 
 }  // namespace vct
