@@ -48,3 +48,32 @@ def test_fragment_list_is_its_halves(cuda, triangles):
             lists.append(passes.svo_fragments(passes.DeviceScene(part), 8, None, passes.light_desc(LIGHT_DIR), sd, ws,
                                               bb_min=whole.bb_min, bb_max=whole.bb_max))
     assert torch.equal(lists[0], torch.cat(lists[1:]))
+
+
+def test_edges_around_the_32_bit_limits(cuda, oracle):
+    """Triangles with edges just below and above 2^17 (512 pixels of 1/256) and edge values past 2^31, fanned with
+    shared edges, at one sample (shadow depth) and eight (opacity at R = 256)."""
+    torch = cuda
+    from vk_voxel_cone_tracing_gb300 import clipmap, passes
+    from vk_voxel_cone_tracing_gb300.scene import _pack
+    rng = np.random.default_rng(4)
+    tris = []
+    for size in (0.5, 3.9, 7.98, 8.0, 8.02, 15.9, 29.0, 300.0):
+        c = rng.uniform(-3, 3, 3) + np.array([0.0, 4.0, 0.0])
+        e = rng.normal(size=(2, 3))
+        e = e / np.linalg.norm(e, axis=1, keepdims=True) * size
+        a, b = c + e[0], c + e[1]
+        tris += [[c, a, a + e[1]], [c, a + e[1], b], [c, b, c - e[0]]]
+    scene = _pack(np.array(tris, np.float32), rng)
+    ds, ws = passes.DeviceScene(scene), passes.Workspace()
+    origin = (-4.0, 16.0, -3.0)
+    depth = torch.empty((2048, 2048), dtype=torch.float32, device="cuda")
+    passes.shadow_depth(ds, passes.light_shadow_desc(origin, LIGHT_DIR), depth, ws)
+    want = oracle.shadow_depth(scene, oracle.light_shadow_desc(origin, LIGHT_DIR), 2048, 2048)
+    assert np.array_equal(depth.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    R = 256
+    regions = clipmap.clip_regions((0.0, 4.0, 0.0), R)
+    atlas = clipmap.new_atlas(R)
+    passes.voxelize_opacity(ds, regions, R, atlas, ws, level_mask=0x5)
+    want = oracle.voxelize_opacity(scene, R, clipmap.regions_to_numpy(regions), level_mask=0x5)
+    assert np.array_equal(atlas.cpu().numpy().view(np.uint32), want)

@@ -334,6 +334,7 @@ struct RasterArgs {
     int levels[6];
     float vp[6][3][16];    // per level, per axis view-projection
     vct_voxelization_desc vd[6];
+    float inv_extent[6];   // clip_image_coords' inv per level
     float pv[16];          // shadow pass: proj * view
     // lighting (injection / SVO)
     TraceParams light;     // light, shadow map and its desc (trace-shared struct)
@@ -534,7 +535,9 @@ __device__ inline bool item_setup(const RasterArgs& A, const WTri& w, int lvl, R
     return rs.ok;
 }
 
-__device__ inline int3 clip_image_coords(const vct_voxelization_desc& d, float3 wp) {
+// `inv`: 1 / clip_max_extent where that is a power of two (the product is then
+// the quotient), else 0.
+__device__ inline int3 clip_image_coords(const vct_voxelization_desc& d, float inv, float3 wp) {
     const float c = d.voxel_size * 0.25f;
     const float lo = d.region_min_corner[0] + c, hi = d.region_max_corner[0] - c;
     float p[3] = {fminf(fmaxf(wp.x, lo), hi), fminf(fmaxf(wp.y, lo), hi), fminf(fmaxf(wp.z, lo), hi)};
@@ -542,7 +545,7 @@ __device__ inline int3 clip_image_coords(const vct_voxelization_desc& d, float3 
     int ic[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float q = p[a] / d.clip_max_extent;
+        float q = inv != 0.0f ? p[a] * inv : p[a] / d.clip_max_extent;
         float f = q - floorf(q);
         ic[a] = ((int)(f * (float)R)) & (R - 1);  // f >= 0 and R a power of two: the value % R
     }
@@ -802,113 +805,124 @@ __host__ __device__ constexpr int sample_y(int s) {
 //   small: every |dX_i|, |dY_i| < 2^17.  A sample of the tile is then within
 //          Mt_i = (|dX_i| + |dY_i|) * 2032 < 2^29 of E_i (offsets < 7 * 256 +
 //          240), so an edge with E_i > Mt_i passes every sample of the tile,
-//          E_i < -Mt_i empties the tile, and the others run in 32 bits;
+//          E_i < -Mt_i empties the tile, and the others run in 32 bits: the
+//          test's e, dx, dy are E_i less 1 where the edge does not own its ties
+//          (covered is then e + ... >= 0) and the deltas, all zero for an edge
+//          that passes, so a sample's test is the sign of three sums or-ed;
 //   zsafe: every vertex depth lies in [0, 1 - 2^-20].  The interpolated depth
 //          of a covered sample is then inside the [0, 1] clip: its weights
 //          are >= 0 and sum to at most (1 + 2^-24)^3 (area = sum of e_i, three
 //          roundings each) and the five roundings of the dot product add at
-//          most a factor (1 + 2^-24)^3, so z <= (1 + 2^-24)^6 (1 - 2^-20) < 1.
-struct TileRegs {
-    long long E[3];     // e_i at the tile corner
-    int dX[3], dY[3];   // small tiles: the edge deltas
-    float z[3], inv_area;
-    uint32_t flags;     // bits 0-2: edge i owns its ties; 3: vertices 1 and 2 swapped;
-                        // 4: small; 5: zsafe; 6-8: edge i passes every sample of the tile
+//          most a factor (1 + 2^-24)^3, so z <= (1 + 2^-24)^6 (1 - 2^-20) < 1;
+//   near:  small and every |E_i| < 2^31 - 2^29, so the tile's edge values fit
+//          32 bits (and convert to float as such).
+constexpr uint32_t kTileSwapped = 8u, kTileSmall = 16u, kTileZsafe = 32u, kTileNear = 64u;  // bits 0-2: edge i owns its ties
+
+struct TileTest {
+    int e[3], dx[3], dy[3];
+    uint32_t flags;
 };
 
 // Per-tile state that the lanes of one warp share: one slot per lane's tile.
 struct TileSlot {
-    TileRegs t;                // the set-up triangle, ready for the per-pixel tests
-    long long dXl[3], dYl[3];  // the edge deltas in 64 bits (tiles that are not small)
+    TileTest test;
+    long long E[3];            // e_i at the tile corner
+    long long dX[3], dY[3];    // the edge deltas
+    float z[3], inv_area;
     int tx, ty, tw;            // tile origin and clipped width in pixels
     uint32_t tw_magic;         // ceil(2^32 / tw) (tw > 1): n / tw = umulhi(n, tw_magic) for n < 64
-    uint32_t px_end;           // inclusive prefix of the warp's tile pixel counts
+    uint32_t px_start, px_end; // the tile's pixels in the warp's list
     uint32_t done;             // covered samples of this tile met in earlier rounds
     uint32_t base, meta;
     uint32_t item;             // the tile's (triangle, level or sub-triangle) item
     float3 p[3], n[3];         // interpolation sources (position, normal)
+    uint32_t pad[2];
 };
+// The lanes read the same field of different slots: a stride of 62 words puts
+// them on 16 banks (64 words: all on one, and the R = 256 hall's opacity pass
+// took 1.40 instead of 0.95 ms; 61 words with the 64-bit fields in halves: 32
+// banks and more loads, 0.64 against 0.59 ms in the shadow pass).
+static_assert(sizeof(TileSlot) == 248, "TileSlot's stride in shared memory");
 
 // Fills the slot's test state for tile (tx, ty); returns false if an edge
 // rejects every sample of the tile.
-__device__ inline bool tile_regs(const RSetup& rs, int tx, int ty, TileSlot& T) {
-    TileRegs& t = T.t;
-    bool small = true;
-    long long Mt[3];
+__device__ inline bool tile_setup(const RSetup& rs, int tx, int ty, TileSlot& T) {
+    bool small = true, near = true;
+    long long E[3], Mt[3];
+    int dX[3], dY[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int a = (i + 1) % 3, c = (i + 2) % 3;
-        const long long dX = rs.X[c] - rs.X[a], dY = rs.Y[c] - rs.Y[a];
-        T.dXl[i] = dX;
-        T.dYl[i] = dY;
-        t.E[i] = dX * ((long long)ty * 256 - rs.Y[a]) - dY * ((long long)tx * 256 - rs.X[a]);
-        const bool si = dX > -(1LL << 17) && dX < (1LL << 17) && dY > -(1LL << 17) && dY < (1LL << 17);
+        const long long dx = rs.X[c] - rs.X[a], dy = rs.Y[c] - rs.Y[a];
+        E[i] = dx * ((long long)ty * 256 - rs.Y[a]) - dy * ((long long)tx * 256 - rs.X[a]);
+        T.E[i] = E[i];
+        T.dX[i] = dx;
+        T.dY[i] = dy;
+        dX[i] = (int)dx;  // meaningful only when small
+        dY[i] = (int)dy;
+        const bool si = dx > -(1LL << 17) && dx < (1LL << 17) && dy > -(1LL << 17) && dy < (1LL << 17);
         small = small && si;
-        t.dX[i] = (int)dX;  // meaningful only when small
-        t.dY[i] = (int)dY;
-        Mt[i] = si ? (llabs(dX) + llabs(dY)) * 2032 : 0;
-        t.z[i] = rs.z[i];
+        near = near && llabs(E[i]) < (1LL << 31) - (1LL << 29);
+        Mt[i] = si ? (llabs(dx) + llabs(dy)) * 2032 : 0;
+        T.z[i] = rs.z[i];
     }
-    uint32_t flags = (uint32_t)rs.owned | (rs.swapped ? 8u : 0u);
+    uint32_t flags = (uint32_t)rs.owned | (rs.swapped ? kTileSwapped : 0u);
     if (small) {
-        flags |= 16u;
+        flags |= kTileSmall | (near ? kTileNear : 0u);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            if (t.E[i] < -Mt[i]) return false;
-            if (t.E[i] > Mt[i]) flags |= 64u << i;
+            if (E[i] < -Mt[i]) return false;
+            const bool pass = E[i] > Mt[i];
+            T.test.e[i] = pass ? 0 : (int)E[i] - (int)!((rs.owned >> i) & 1);
+            T.test.dx[i] = pass ? 0 : dX[i];
+            T.test.dy[i] = pass ? 0 : dY[i];
         }
     }
     const float zhi = 0.99999904632568359375f;  // 1 - 2^-20
     if (rs.z[0] >= 0.0f && rs.z[1] >= 0.0f && rs.z[2] >= 0.0f && rs.z[0] <= zhi && rs.z[1] <= zhi && rs.z[2] <= zhi)
-        flags |= 32u;
-    t.flags = flags;
-    t.inv_area = rs.inv_area;
+        flags |= kTileZsafe;
+    T.test.flags = flags;
+    T.inv_area = rs.inv_area;
     return true;
 }
 
 // Barycentrics and depth of the sample at offset (ox, oy) from the tile
 // corner: the pinned FP32 barycentrics and depth.
-__device__ inline void sample_bz(const TileRegs& t, const TileSlot& T, int ox, int oy, float b[3], float& z) {
+__device__ inline void sample_bz(const TileSlot& T, int ox, int oy, float b[3], float& z) {
+    const uint32_t flags = T.test.flags;
     float bo[3];
+    if (flags & kTileNear) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const long long e = (t.flags & 16u) ? t.E[i] + (long long)(t.dX[i] * oy - t.dY[i] * ox)
-                                            : t.E[i] + (T.dXl[i] * oy - T.dYl[i] * ox);
-        bo[i] = (float)e * t.inv_area;
+        for (int i = 0; i < 3; ++i)
+            bo[i] = (float)((int)T.E[i] + ((int)T.dX[i] * oy - (int)T.dY[i] * ox)) * T.inv_area;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) bo[i] = (float)(T.E[i] + (T.dX[i] * oy - T.dY[i] * ox)) * T.inv_area;
     }
-    z = (bo[0] * t.z[0] + bo[1] * t.z[1]) + bo[2] * t.z[2];
+    z = (bo[0] * T.z[0] + bo[1] * T.z[1]) + bo[2] * T.z[2];
     b[0] = bo[0];
-    b[1] = (t.flags & 8u) ? bo[2] : bo[1];
-    b[2] = (t.flags & 8u) ? bo[1] : bo[2];
+    b[1] = (flags & kTileSwapped) ? bo[2] : bo[1];
+    b[2] = (flags & kTileSwapped) ? bo[1] : bo[2];
 }
 
 // Coverage mask of the NS samples of the pixel at offset (ox0, oy0) from the
 // tile corner (bit s: sample s covered and inside the depth clip).
 template <int NS>
-__device__ inline uint32_t cover_pixel(const TileRegs& t, const TileSlot& T, int ox0, int oy0) {
+__device__ inline uint32_t cover_pixel(const TileTest& t, const TileSlot& T, int ox0, int oy0) {
     uint32_t mask = 0;
-    if (t.flags & 16u) {
+    if (t.flags & kTileSmall) {
         int base[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) base[i] = (int)t.E[i] + (t.dX[i] * oy0 - t.dY[i] * ox0);
+        for (int i = 0; i < 3; ++i) base[i] = t.e[i] + (t.dx[i] * oy0 - t.dy[i] * ox0);
 #pragma unroll
-        for (int s = 0; s < NS; ++s) {
+        for (int s = NS - 1; s >= 0; --s) {
             const int ox = NS == 1 ? 128 : sample_x(s), oy = NS == 1 ? 128 : sample_y(s);
-            bool cov = true;
+            int x = 0;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                if (!((t.flags >> (6 + i)) & 1u)) {
-                    const int e = base[i] + (t.dX[i] * oy - t.dY[i] * ox);
-                    cov = cov && (e > 0 || (e == 0 && ((t.flags >> i) & 1u)));
-                }
-            }
-            if (cov && !(t.flags & 32u)) {
-                float b[3], z;
-                sample_bz(t, T, ox0 + ox, oy0 + oy, b, z);
-                cov = z >= 0.0f && z <= 1.0f;
-            }
-            mask |= (uint32_t)cov << s;
+            for (int i = 0; i < 3; ++i) x |= base[i] + (t.dx[i] * oy - t.dy[i] * ox);
+            mask = __funnelshift_l((uint32_t)x, mask, 1);  // the sign bit in: 1 = outside
         }
+        mask = ~mask & ((1u << NS) - 1u);
     } else {
 #pragma unroll 1
         for (int s = 0; s < NS; ++s) {
@@ -916,24 +930,21 @@ __device__ inline uint32_t cover_pixel(const TileRegs& t, const TileSlot& T, int
             bool cov = true;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                const long long e = t.E[i] + (T.dXl[i] * oy - T.dYl[i] * ox);
+                const long long e = T.E[i] + (T.dX[i] * oy - T.dY[i] * ox);
                 cov = cov && (e > 0 || (e == 0 && ((t.flags >> i) & 1u)));
-            }
-            if (cov) {
-                float b[3], z;
-                sample_bz(t, T, ox, oy, b, z);
-                cov = z >= 0.0f && z <= 1.0f;
             }
             mask |= (uint32_t)cov << s;
         }
     }
+    if (!(t.flags & kTileZsafe))
+        for (uint32_t m = mask; m; m &= m - 1u) {
+            const int s = __ffs(m) - 1;
+            float b[3], z;
+            sample_bz(T, ox0 + (NS == 1 ? 128 : c_sample_loc8[s][0]), oy0 + (NS == 1 ? 128 : c_sample_loc8[s][1]), b, z);
+            if (!(z >= 0.0f && z <= 1.0f)) mask &= ~(1u << s);
+        }
     return mask;
 }
-
-// Per-sample work of the coverage kernels (opacity stores, fragment
-// emission) over the round's covered samples dealt one per lane (true), or
-// over each lane's own pixel mask (false).
-constexpr bool kDealCoveredSamples = true;
 
 // The covered samples of a warp's 32 pixels (lane i's pixel has coverage
 // mask `mask`), dealt one per lane in (pixel, sample) order, 32 per round:
@@ -999,9 +1010,15 @@ static int chunk_group(bool one_sample, uint32_t tiles) {
 // (chunk_tile) -- one per lane -- sets each up once into shared memory, then
 // flattens the (tile, pixel) pairs of all 32 tiles and walks them 32 at a
 // time, one pixel (all of its samples) per lane, so every lane does the same
-// work however unequal the tiles are.  Pixel q of the flattened list belongs
-// to the first tile whose inclusive pixel sum exceeds q; within a tile pixels
-// are row-major, so the list is in traversal order (item, tile, pixel, sample).
+// work however unequal the tiles are.  Within a tile pixels are row-major, so a
+// tile's samples are met in traversal order (pixel, sample).  A round's lanes
+// find their pixels' tiles from the mask of the tiles that start in it (one
+// warp reduction); the work per pixel is the test of its samples against three
+// edges, which bounds the kernel on small triangles.  With the sign-bit tests,
+// 32-bit edge values, the reduction instead of a binary search per pixel and
+// the slots' stride: 1M-triangle hall at R = 256, opacity + count 1.76 -> 0.95
+// ms, emission 0.85 -> 0.51, shadow 0.81 -> 0.59; octree count and emission of
+// the 4M-triangle terrain 1.12 -> 0.53 and 1.48 -> 1.01 ms.
 //   P_DIRECT writes the pass's output (opacity, shadow depth, atomic injection);
 //   P_COUNT counts covered samples and their records per tile;
 //   P_WRITE emits one FragDesc per covered sample at its rank within the tile
@@ -1016,9 +1033,12 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
     constexpr int NS = (KIND == K_SHADOW || KIND == K_GBUFFER) ? 1 : 8;
     constexpr bool RANKED = PHASE != P_DIRECT;
     // the opacity writes run over the round's covered samples dealt to the lanes
-    constexpr bool FLAT_OPACITY = kDealCoveredSamples && (KIND == K_OPACITY || KIND == K_OPA_COUNT) && PHASE != P_WRITE;
+    constexpr bool FLAT_OPACITY = (KIND == K_OPACITY || KIND == K_OPA_COUNT) && PHASE != P_WRITE;
+    // the normals are read where samples are shaded or emitted
+    constexpr bool NORMALS = PHASE == P_WRITE || (KIND == K_INJECT && PHASE == P_DIRECT);
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ TileSlot slots[4][32];
+    __shared__ uint8_t nonempty[4][32];  // the warp's tiles with pixels, in order
     const int lane = threadIdx.x & 31;
     TileSlot* S = slots[threadIdx.x >> 5];
     const uint32_t* __restrict__ tile_end = plan.tile_end;
@@ -1052,7 +1072,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                 const int tcols = ((rs.px1 - rs.px0) >> 3) + 1;
                 const int tx = rs.px0 + 8 * (int)(local % (uint32_t)tcols), ty = rs.py0 + 8 * (int)(local / (uint32_t)tcols);
                 const int tw = min(tx + 7, rs.px1) - tx + 1, th = min(ty + 7, rs.py1) - ty + 1;
-                npx = tile_regs(rs, tx, ty, T) ? (uint32_t)(tw * th) : 0u;
+                npx = tile_setup(rs, tx, ty, T) ? (uint32_t)(tw * th) : 0u;
                 T.tx = tx;
                 T.ty = ty;
                 T.tw = tw;
@@ -1063,7 +1083,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         T.p[k] = KIND == K_SVO ? pos[k] : w.p[k];
-                        T.n[k] = w.n[k];
+                        if (NORMALS) T.n[k] = w.n[k];
                     }
                 }
                 if (PHASE == P_WRITE) T.base = (uint32_t)offs[g];
@@ -1076,11 +1096,14 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
             const uint32_t v = __shfl_up_sync(FULL, incl, d);
             if (lane >= d) incl += v;
         }
+        S[lane].px_start = incl - npx;
         S[lane].px_end = incl;
         S[lane].done = 0u;
+        const unsigned filled = __ballot_sync(FULL, npx != 0u);
+        if (npx) nonempty[threadIdx.x >> 5][__popc(filled & ((1u << lane) - 1u))] = (uint8_t)lane;
         const uint32_t P = __shfl_sync(FULL, incl, 31);
         __syncwarp();
-        TileRegs t;
+        TileTest t;
         int cj = -1;
         if (KIND == K_SHADOW || KIND == K_GBUFFER) {
             // one centre sample per pixel: each lane takes four consecutive
@@ -1097,16 +1120,15 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                 for (uint32_t q = q0; q < q0 + 4u && q < P; ++q) {
                     while (S[j].px_end <= q) ++j;  // the next pixel's tile (at most 3 steps)
                     if (j != cj) {
-                        t = S[j].t;
+                        t = S[j].test;
                         cj = j;
                     }
-                    const uint32_t start = j > 0 ? S[j - 1].px_end : 0u;
-                    const uint32_t lp = q - start, tw = (uint32_t)S[j].tw;
+                    const uint32_t lp = q - S[j].px_start, tw = (uint32_t)S[j].tw;
                     const uint32_t row = tw > 1u ? __umulhi(lp, S[j].tw_magic) : lp;
                     const int ox0 = (int)(lp - row * tw) * 256, oy0 = (int)row * 256;
                     if (cover_pixel<1>(t, S[j], ox0, oy0)) {
                         float b[3], z;
-                        sample_bz(t, S[j], ox0 + 128, oy0 + 128, b, z);
+                        sample_bz(S[j], ox0 + 128, oy0 + 128, b, z);
                         const int px = S[j].tx + (ox0 >> 8), py = S[j].ty + (oy0 >> 8);
                         if (KIND == K_SHADOW) {
                             atomicMin(reinterpret_cast<unsigned int*>(A.depth) + (int64_t)py * A.W + px,
@@ -1122,70 +1144,46 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
             __syncwarp();
             continue;
         }
+        uint32_t begun = 0;  // tiles that start before the round
         for (uint32_t q0 = 0; q0 < P; q0 += 32u) {
             const uint32_t q = q0 + lane;
             const bool act = q < P;
+            const uint32_t first_px = incl - npx - q0;  // wraps for tiles that start before q0
+            const uint32_t heads = __reduce_or_sync(FULL, npx && first_px < 32u ? 1u << first_px : 0u);
+            const uint32_t ord = begun + (uint32_t)__popc(heads & (0xffffffffu >> (31 - lane)));
+            begun += (uint32_t)__popc(heads);
             int j = 0;
             uint32_t start = 0, mask = 0;
-            int px = 0, py = 0, ox0 = 0, oy0 = 0;
+            int ox0 = 0, oy0 = 0;
             if (act) {
-                int lo = 0, hi = 31;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (S[mid].px_end > q) hi = mid;
-                    else lo = mid + 1;
-                }
-                j = lo;
-                start = j > 0 ? S[j - 1].px_end : 0u;
+                j = nonempty[threadIdx.x >> 5][ord - 1u];
+                start = S[j].px_start;
                 if (j != cj) {
-                    t = S[j].t;
+                    t = S[j].test;
                     cj = j;
                 }
                 const uint32_t lp = q - start, tw = (uint32_t)S[j].tw;
                 const uint32_t row = tw > 1u ? __umulhi(lp, S[j].tw_magic) : lp;
                 ox0 = (int)(lp - row * tw) * 256;
                 oy0 = (int)row * 256;
-                px = S[j].tx + (ox0 >> 8);
-                py = S[j].ty + (oy0 >> 8);
                 mask = cover_pixel<NS>(t, S[j], ox0, oy0);
-                if (!FLAT_OPACITY && (PHASE == P_DIRECT || KIND == K_OPA_COUNT) && mask) {
+                if (KIND == K_INJECT && PHASE == P_DIRECT) {
                     const TileSlot& T = S[j];
                     const int lvl = (int)(T.meta & 7u);
-                    int3 last_ic = make_int3(-1, -1, -1);  // opacity: the previous sample's voxel (stores are idempotent)
                     for (uint32_t m = mask; m; m &= m - 1u) {
                         const int s = __ffs(m) - 1;
                         float b[3], z;
-                        sample_bz(t, T, ox0 + (NS == 1 ? 128 : c_sample_loc8[s][0]),
-                                  oy0 + (NS == 1 ? 128 : c_sample_loc8[s][1]), b, z);
-                        if (KIND == K_SHADOW) {
-                            atomicMin(reinterpret_cast<unsigned int*>(A.depth) + (int64_t)py * A.W + px, __float_as_uint(z));
-                        } else if (KIND == K_OPACITY || KIND == K_OPA_COUNT) {
-                            const vct_voxelization_desc& d = A.vd[lvl];
-                            const float3 wp = interp3(b, T.p);
-                            if (wp.x < d.region_min_corner[0] || wp.y < d.region_min_corner[1] ||
-                                wp.z < d.region_min_corner[2] || wp.x > d.region_max_corner[0] ||
-                                wp.y > d.region_max_corner[1] || wp.z > d.region_max_corner[2])
-                                continue;
-                            if (((A.slab_levels >> lvl) & 1u) && !in_slabs(A, lvl, wp)) continue;
-                            const AtlasDims AD(A.R);
-                            const int3 ic = clip_image_coords(d, wp);
-                            if (ic.x == last_ic.x && ic.y == last_ic.y && ic.z == last_ic.z) continue;
-                            last_ic = ic;
-                            if (A.opa_bits) mark_voxel(A.opa_bits, A.R, lvl, ic);
-                            else
-                                for (int f = 0; f < 6; ++f) A.atlas[AD.index(ic.x + (A.R + 2) * f, ic.y, ic.z)] = 0xFFFFFFFFu;
-                        } else if (KIND == K_INJECT) {
-                            const vct_gltf_shade_material mat = material_of(A.s, T.meta >> 3);
-                            const float3 wp = interp3(b, T.p);
-                            const InjLight L = inject_light(A, mat, wp, interp3(b, T.n));
-                            const int3 ic = clip_image_coords(A.vd[lvl], wp);
-                            uint32_t* cell = A.atlas + AtlasDims(A.R).index(ic.x, ic.y, ic.z);
-                            for (int f = 0; f < 6; ++f) {
-                                const bool odd = (L.flags >> (2 + f / 2)) & 1u;
-                                if (!(L.flags & kInjLit) || (!(L.flags & kInjEmissive) && odd != (bool)(f & 1))) continue;
-                                const float3 v = inject_value(make_float3(L.c[0], L.c[1], L.c[2]), L.w[f / 2], L.flags);
-                                rgba8_avg_atomic(cell + (A.R + 2) * f, v.x, v.y, v.z, 1.0f, err);
-                            }
+                        sample_bz(T, ox0 + c_sample_loc8[s][0], oy0 + c_sample_loc8[s][1], b, z);
+                        const vct_gltf_shade_material mat = material_of(A.s, T.meta >> 3);
+                        const float3 wp = interp3(b, T.p);
+                        const InjLight L = inject_light(A, mat, wp, interp3(b, T.n));
+                        const int3 ic = clip_image_coords(A.vd[lvl], A.inv_extent[lvl], wp);
+                        uint32_t* cell = A.atlas + AtlasDims(A.R).index(ic.x, ic.y, ic.z);
+                        for (int f = 0; f < 6; ++f) {
+                            const bool odd = (L.flags >> (2 + f / 2)) & 1u;
+                            if (!(L.flags & kInjLit) || (!(L.flags & kInjEmissive) && odd != (bool)(f & 1))) continue;
+                            const float3 v = inject_value(make_float3(L.c[0], L.c[1], L.c[2]), L.w[f / 2], L.flags);
+                            rgba8_avg_atomic(cell + (A.R + 2) * f, v.x, v.y, v.z, 1.0f, err);
                         }
                     }
                 }
@@ -1203,7 +1201,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                         const TileSlot& T = S[jo];
                         const int lvl = (int)(T.meta & 7u);
                         float b[3], z;
-                        sample_bz(T.t, T, oxo + c_sample_loc8[s][0], oyo + c_sample_loc8[s][1], b, z);
+                        sample_bz(T, oxo + c_sample_loc8[s][0], oyo + c_sample_loc8[s][1], b, z);
                         const vct_voxelization_desc& d = A.vd[lvl];
                         const float3 wp = interp3(b, T.p);
                         const bool inside = !(wp.x < d.region_min_corner[0] || wp.y < d.region_min_corner[1] ||
@@ -1211,7 +1209,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                                               wp.y > d.region_max_corner[1] || wp.z > d.region_max_corner[2]) &&
                                             !(((A.slab_levels >> lvl) & 1u) && !in_slabs(A, lvl, wp));
                         if (inside) {
-                            ic = clip_image_coords(d, wp);
+                            ic = clip_image_coords(d, A.inv_extent[lvl], wp);
                             keep = true;
                         }
                     }
@@ -1245,25 +1243,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                 __syncwarp();
                 if (last) S[j].done += ci - cx_first;
                 __syncwarp();
-                if constexpr (PHASE == P_WRITE && !kDealCoveredSamples) {
-                    if (mask) {
-                        const TileSlot& T = S[j];
-                        uint32_t k = rank;
-                        for (uint32_t m = mask; m; m &= m - 1u) {
-                            const int s = __ffs(m) - 1;
-                            float b[3], z;
-                            sample_bz(t, T, ox0 + c_sample_loc8[s][0], oy0 + c_sample_loc8[s][1], b, z);
-                            const float3 p = interp3(b, T.p);
-                            const float3 nn = interp3(b, T.n);
-                            FragDesc d;
-                            d.p = make_float4(p.x, p.y, p.z, __uint_as_float(T.meta));
-                            d.n = make_float4(nn.x, nn.y, nn.z, 0.0f);
-                            frags[T.base + k] = d;
-                            ++k;
-                        }
-                    }
-                }
-                if constexpr (PHASE == P_WRITE && kDealCoveredSamples) {
+                if constexpr (PHASE == P_WRITE) {
                     // the r-th covered sample of a pixel goes to its tile's slot rank + r
                     for_each_covered(mask, lane, [&](bool valid, int o, int s, uint32_t r) {
                         const int jo = __shfl_sync(FULL, j, o), oxo = __shfl_sync(FULL, ox0, o),
@@ -1272,7 +1252,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                         if (valid) {
                             const TileSlot& T = S[jo];
                             float b[3], z;
-                            sample_bz(T.t, T, oxo + c_sample_loc8[s][0], oyo + c_sample_loc8[s][1], b, z);
+                            sample_bz(T, oxo + c_sample_loc8[s][0], oyo + c_sample_loc8[s][1], b, z);
                             const float3 p = interp3(b, T.p);
                             const float3 nn = interp3(b, T.n);
                             FragDesc d;
@@ -1344,7 +1324,7 @@ __global__ void __launch_bounds__(256) k_inject_shade(const __grid_constant__ Ra
             const uint32_t meta = __float_as_uint(d.p.w);
             const float3 wp = make_float3(d.p.x, d.p.y, d.p.z);
             const vct_voxelization_desc& vd = A.vd[meta & 7u];
-            const int3 ic = clip_image_coords(vd, wp);
+            const int3 ic = clip_image_coords(vd, A.inv_extent[meta & 7u], wp);
             const Key y = (Key)(ic.y - 1 - (A.R + 2) * (int)vd.clip_level);
             key = (((Key)vd.clip_level * R + (Key)(ic.z - 1)) * R + y) * R + (Key)(ic.x - 1);
             keys[f] = key;
@@ -2116,6 +2096,9 @@ static void fill_clipmap_levels(RasterArgs& A, const vct_clipmap_region* regions
     for (int l = 0; l < 6; ++l) {
         voxel_view_proj(regions[l], &A.vp[l][0][0]);
         A.vd[l] = voxelization_desc(regions, l, R);
+        int e = 0;
+        const bool pow2 = frexpf(A.vd[l].clip_max_extent, &e) == 0.5f && e > -100 && e < 100;
+        A.inv_extent[l] = pow2 ? 1.0f / A.vd[l].clip_max_extent : 0.0f;
         if ((level_mask >> l) & 1u) A.levels[A.nlevels++] = l;
     }
 }
@@ -2743,7 +2726,6 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
                         cudaSurfaceObject_t mirror, FrameBits* bits_out, cudaStream_t st) {
     const int R = f->clipmap_resolution;
-    void* stream = st;
     int rc;
     const bool toroidal = nslabs >= 0;
     SlabPlan P;
