@@ -91,19 +91,6 @@ __device__ __forceinline__ uint2 svo_nodes(const SvoScene& S, float3 p, uint32_t
     return make_uint2(vlo, vhi);
 }
 
-// ceil(log2(|center - pos| / min_radius)) from the squared distance: with
-// t = (dist / radius)^2 up to a few ulp, ceil(log2(t) / 2) is an exponent
-// unless t is next to an even power of two, where the shader's expression
-// decides (its logarithm is within an ulp, which moves no other ceil).
-__device__ __forceinline__ float svo_min_level(const SvoScene& S, float3 center, float3 pos) {
-    const float d2 = dot3(center - pos, center - pos);
-    const uint32_t bits = __float_as_uint(d2 * S.inv_r2);
-    const int rel = (int)(bits - 0x3f800000u);  // even powers of two are multiples of 2^24
-    if (((uint32_t)(rel + 128) & 0xffffffu) < 256u || bits - 0x0d800000u >= 0x64800000u)
-        return ceilf(log2f(sqrtf(d2) / S.min_radius));
-    return (float)((rel >> 24) + 1);
-}
-
 __device__ __forceinline__ float svo_over_uvs(const SvoScene& S, float x, float uvs) {
     return S.uvs_pow2 ? x * S.inv_uvs : x / uvs;
 }
@@ -121,7 +108,7 @@ __device__ float4 svo_trace_cone(const SvoScene& S, const vct_cone_tracing_desc&
     int k = 0;
     while (step < kMaxTraceDistance && occlusion < 1.0f) {
         const float3 pos = start + dir * step;
-        const float min_level = svo_min_level(S, center, pos);
+        const float min_level = cone_min_level(S.inv_r2, S.min_radius, center, pos);
         float cur_level;
         if (k < levels) cur_level = level_at[k];
         else cur_level = log2f(svo_over_uvs(S, diameter, uvs));

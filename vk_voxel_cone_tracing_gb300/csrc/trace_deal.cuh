@@ -42,9 +42,8 @@ struct DealArgs {
 // 32 / 16 / 8 / 4 samples per item): 4096 samples 115 / 74 / 70 / 67, 16,384
 // samples 171 / 146 / 149 / 153, 65,536 samples 316 / 325 / 337 / 352; so the
 // texture form fills 6 warps per SM (its specular kernel runs beside it).  The
-// exact form alone on the chip: 65,536 samples 3344 / 3151 / 3127 / 3189,
-// 131,072 samples 4241 / 4146 / 4226 / 4387, 262,144 samples 6272 / 6389 /
-// 6751: 32 warps per SM.
+// exact form alone on the chip: 65,536 samples 1167 / 1145 / 1161 at 16 / 8 / 4
+// (16 / 32 / 64 warps per SM): 32 warps per SM.
 inline int deal_samples_per_warp(int64_t n, int64_t warps) {
     int s = 32;
     while (s > 4 && (n + s - 1) / s < warps) s >>= 1;

@@ -7,12 +7,20 @@
 // -fmad=false so no multiply-add is fused.  The work is laid out like the
 // texture form's: samples in a coherent order (normal class, then Morton),
 // the diffuse cones of 32 samples dealt to the lanes of a warp
-// (trace_deal.cuh), each cone marched by trace_cone; the specular cones one
-// per lane over a list grouped by aperture (so a warp's cones march nearly
-// the same number of steps).  The specular cone is traced wherever the
-// shader traces it (every rendering mode), the diffuse cones likewise.
+// (trace_deal.cuh), each cone marched by trace_cone; the specular cones over a
+// list grouped by aperture (so a warp's cones march nearly the same number of
+// steps), one or more lanes to a cone.  The specular cone is traced wherever
+// the shader traces it (every rendering mode), the diffuse cones likewise.
+//
+// What bounds it: instructions (57 a texel before the packed lerps, the
+// two-instruction decode and the known divisors of trace_exact.cuh, 25 now;
+// half the issue slots are still lost to fetching the loop's code) and, for
+// the specular cones, the length of the longest march: 65,536 cones on one
+// lane each are 13 warps an SM, nearly all of them done when the longest are
+// half way.  65,536 samples on the R = 128 room went from 3.48 to 1.15 ms
+// (diffuse 1.03 to 0.5, specular 2.37 to 0.5), the float form's from 1.60 to
+// 0.67 ms, every output unchanged.
 #include <cstring>
-#include <type_traits>
 
 #include <cub/cub.cuh>
 
@@ -24,79 +32,144 @@ namespace vct {
 constexpr int kExactWarps = 4;  // warps per block of the diffuse kernel
 constexpr int kExactDiffuseWarpsPerSm = 32;  // warp items per SM that deal_samples_per_warp aims at
 
-// Tickets (work to warps as they free up) for the texture and float reads;
-// the linear RGBA8 atlas's loads run faster with the static deal.
-template <class Atlas>
-constexpr bool kExactTickets = !std::is_same<Atlas, ExactAtlas>::value;
+constexpr int kExactLevels = 128;  // steps of the diffuse schedule kept as a table (default descriptors take 19 to 40)
 
 template <class Atlas>
 struct ExactDiffuseMarch {
-    Atlas T;
-    const vct_cone_tracing_desc* d;
-    float aperture, step_factor;
+    const Atlas& T;
+    const MarchScale& C;
+    const vct_cone_tracing_desc& d;
+    float coef, step_factor;
+    const float* level_at;
+    int levels;
     __device__ __forceinline__ float4 operator()(float3 start, float3 dir, float start_level,
                                                  unsigned long long& steps) const {
-        return trace_cone(T, *d, start, dir, aperture, kMaxTraceDistance, start_level, step_factor, steps);
+        return trace_cone(T, C, d, make_cone(d, start, dir, coef, start_level, step_factor), kMaxTraceDistance,
+                          level_at, levels, steps);
     }
 };
 
 template <class Atlas>
-__global__ void __launch_bounds__(32 * kExactWarps) k_exact_diffuse(TraceParams P, Atlas T,
+__global__ void __launch_bounds__(32 * kExactWarps) k_exact_diffuse(const __grid_constant__ TraceParams P,
+                                                                    const __grid_constant__ MarchScale C,
+                                                                    const __grid_constant__ Atlas T,
                                                                     const vct_surface_sample* __restrict__ samples,
                                                                     int64_t n, const uint32_t* __restrict__ order,
                                                                     float* __restrict__ dout, float* __restrict__ sout,
                                                                     unsigned long long* __restrict__ step_counter,
                                                                     unsigned int* __restrict__ ticket, int per_warp) {
+    __shared__ float s_level[kExactLevels];
+    __shared__ int s_levels;
     const bool c32 = P.d.enable_32_cones != 0;
+    ConeGeo K;  // the schedule's part of every diffuse cone: it is the same for all of them
+    K.uvs = P.d.voxel_size;
+    K.coef = cone_coef(P.diffuse_aperture);
+    K.step_factor = fmaxf(kMinTraceStepFactor, P.d.min_trace_step_factor);
+    K.start_level = 0.0f;
+    if (threadIdx.x == 0) {
+        Sched s = first_sched(K);
+        int k = 0;
+        for (; k < kExactLevels && s.step < kMaxTraceDistance; ++k) {
+            s_level[k] = s.diameter;
+            sched_advance(s, K);
+        }
+        s_levels = k;
+    }
+    __syncthreads();
+    const int levels = s_levels;
+    for (int k = threadIdx.x; k < levels; k += blockDim.x) s_level[k] = cone_raw_level(C, s_level[k], K.uvs);
+    __syncthreads();
     DealArgs D{&P, samples, n, order, 0u, (uint32_t)n, dout, sout, c32 ? 32 : 16, true, true, per_warp};
-    const ExactDiffuseMarch<Atlas> march{T, &P.d, P.diffuse_aperture,
-                                         fmaxf(kMinTraceStepFactor, P.d.min_trace_step_factor)};
+    const ExactDiffuseMarch<Atlas> march{T, C, P.d, K.coef, K.step_factor, s_level, levels};
     unsigned long long steps = 0;
-    deal_diffuse<kExactWarps, kExactTickets<Atlas>>(D, march, steps, ticket);
+    deal_diffuse<kExactWarps, true>(D, march, steps, ticket);
     add_steps(step_counter, steps);
 }
 
-// One lane per specular cone of the list.  The list is grouped by aperture
-// (then kept in the coherent order), and a cone's step count depends only on
-// its aperture (and the occlusion stop), so a warp's cones march in step.
+// Lanes per specular cone: a power of two up to kExactMaxGroup, as few as give
+// kExactSpecWarpsPerSm warps per SM.  Measured (whole trace, 65,536 cones, us):
+// two lanes 1,485, four 1,145, eight 1,154; every further lane repeats the
+// additions, so larger lists take fewer.
+constexpr int kExactMaxGroup = 8;
+constexpr int kExactSpecWarpsPerSm = 32;
+
+// One group of `group` lanes per specular cone of the list.  The list is
+// grouped by aperture (then kept in the coherent order), and a cone's step
+// count depends only on its aperture (and the occlusion stop), so a warp's
+// cones march in step; 32 / group consecutive cones go to a warp at a time as
+// warps free up, the longest first.  The group's lanes take consecutive steps:
+// each samples its own, then all add the terms in step order, so every cone's
+// sum is the one-lane march's bit for bit (the steps after the occlusion stop
+// are dropped).
 template <class Atlas>
-__global__ void __launch_bounds__(128) k_exact_specular(TraceParams P, Atlas T,
+__global__ void __launch_bounds__(128) k_exact_specular(const __grid_constant__ TraceParams P,
+                                                        const __grid_constant__ MarchScale C,
+                                                        const __grid_constant__ Atlas T,
                                                         const vct_surface_sample* __restrict__ samples,
                                                         const uint32_t* __restrict__ list,
                                                         const unsigned int* __restrict__ spec_count,
                                                         float* __restrict__ sout,
                                                         unsigned long long* __restrict__ step_counter,
                                                         unsigned int* __restrict__ ticket) {
+    constexpr unsigned kFull = 0xffffffffu;
     const vct_cone_tracing_desc& d = P.d;
     const int64_t m = *spec_count;
     const int lane = threadIdx.x & 31;
+    int group = 1;
+    while (group < kExactMaxGroup && m * group < (int64_t)gridDim.x * 128) group <<= 1;
+    const int cones = 32 / group, first = lane & ~(group - 1);
+    const uint32_t firsts = group == 1 ? kFull : (group == 2 ? 0x55555555u : (group == 4 ? 0x11111111u : 0x01010101u));
     unsigned long long steps = 0;
-    // with tickets, 32 consecutive cones of the list to the warp at a time as warps free up; without, a
-    // static grid stride
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t c_static = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - stride;
     for (;;) {
-        int64_t c;
-        if constexpr (kExactTickets<Atlas>) {
-            uint32_t c0 = 0;
-            if (lane == 0) c0 = atomicAdd(ticket, 32u);
-            c0 = __shfl_sync(0xffffffffu, c0, 0);
-            if ((int64_t)c0 >= m) break;
-            c = (int64_t)c0 + lane;
-            if (c >= m) continue;
-        } else {
-            c_static += stride;
-            if (c_static >= m) break;
-            c = c_static;
-        }
-        const uint32_t idx = __ldg(list + c);
+        uint32_t c0 = 0;
+        if (lane == 0) c0 = atomicAdd(ticket, (unsigned)cones);
+        c0 = __shfl_sync(kFull, c0, 0);
+        if ((int64_t)c0 >= m) break;
+        const int64_t c = (int64_t)c0 + lane / group;
+        const bool valid = c < m;
+        const uint32_t idx = __ldg(list + (valid ? c : (int64_t)c0));
         const GSample g = load_sample(samples + idx, P.eye);
         const float min_level = calc_min_level(d, g.wp);
         const float vs = d.voxel_size * exp2f(min_level);
         const float3 start = g.wp + g.normal * (vs * d.trace_start_offset);
         const float3 sdir = reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal);
-        const float4 r = trace_cone(T, d, start, sdir, fmaxf(g.roughness, kMinSpecularAperture), kMaxTraceDistance,
-                                    min_level, d.voxel_size, steps);
+        const ConeGeo K = make_cone(d, start, sdir, cone_coef(fmaxf(g.roughness, kMinSpecularAperture)), min_level,
+                                    d.voxel_size);
+        ConeSum sum{make_float4(0.f, 0.f, 0.f, 0.f), 0.0f};
+        Sched s = first_sched(K);  // the group's next unsampled step, the same on its lanes
+        bool running = valid && s.step < kMaxTraceDistance;
+        unsigned int taken = 0;
+        while (__any_sync(kFull, running)) {
+            Sched mine = s;
+            for (int j = 0; j < group; ++j) {
+                if (lane - first == j) mine = s;
+                sched_advance(s, K);
+            }
+            const bool has = running && mine.step < kMaxTraceDistance;
+            StepTerm t;
+            t.some = false;
+            if (has)
+                t = exact_step(T, C, d, K, mine.step, mine.seg, cone_raw_level(C, mine.diameter, K.uvs));
+            const uint32_t has_mask = __ballot_sync(kFull, has) >> first, some = __ballot_sync(kFull, t.some);
+            if (some == 0u) {  // nothing to add in the warp
+                taken += __popc(has_mask & ((2u << (group - 1)) - 1u));
+            } else {
+                for (int j = 0; j < group; ++j) {
+                    const bool on = ((has_mask >> j) & 1u) && sum.occlusion < 1.0f;
+                    taken += on;
+                    if (!((some >> j) & firsts)) continue;  // no cone of the warp adds at its step j
+                    const int src = first + j;
+                    const float3 rc = f3(__shfl_sync(kFull, t.c.x, src), __shfl_sync(kFull, t.c.y, src),
+                                         __shfl_sync(kFull, t.c.z, src));
+                    const float op = __shfl_sync(kFull, t.op, src), q = __shfl_sync(kFull, t.q, src);
+                    if (on && ((some >> src) & 1u)) sum.add(rc, op, q);
+                }
+            }
+            running = running && s.step < kMaxTraceDistance && sum.occlusion < 1.0f;
+        }
+        if (lane != first || !valid) continue;
+        steps += taken;
+        const float4 r = sum.result();
         const float isi = d.indirect_specular_intensity;
         const uint32_t mode = d.rendering_mode;
         float4 S = make_float4(0.f, 0.f, 0.f, 1.f);  // write_outputs' specular output
@@ -326,6 +399,7 @@ template <class Atlas>
 static int launch_exact(const TraceParams& P, const Atlas& T, const vct_surface_sample* samples, int64_t n,
                         float* dout, float* sout, unsigned long long* cone_steps, cudaStream_t st) {
     constexpr int64_t kChunk = 1LL << 30;
+    const MarchScale C = march_scale(P.d);
     for (int64_t off = 0; off < n; off += kChunk) {
         const int64_t m = n - off < kChunk ? n - off : kChunk;
         const vct_surface_sample* smp = samples + off;
@@ -337,12 +411,12 @@ static int launch_exact(const TraceParams& P, const Atlas& T, const vct_surface_
         const int per_warp = deal_samples_per_warp(m, 152 * kExactDiffuseWarpsPerSm);
         const int64_t gdw = (m + (int64_t)per_warp * kExactWarps - 1) / ((int64_t)per_warp * kExactWarps);
         k_exact_diffuse<<<(int)(gdw > 152 * 16 ? 152 * 16 : gdw), 32 * kExactWarps, 0, st>>>(
-            P, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket, per_warp);
+            P, C, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            const int64_t gl = (m + 127) / 128;
-            k_exact_specular<<<(int)(gl > 152 * 16 ? 152 * 16 : gl), 128, 0, st>>>(
-                P, T, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, spec_ticket);
+            const int64_t gl = (m * kExactMaxGroup + 127) / 128, full = 152 * kExactSpecWarpsPerSm / 4;
+            k_exact_specular<<<(int)(gl > full ? full : gl), 128, 0, st>>>(
+                P, C, T, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, spec_ticket);
             e = cudaGetLastError();
         }
         exact_plan_free(&plan, st);

@@ -100,34 +100,28 @@ __device__ __forceinline__ void texture3d_grad(float4* __restrict__ G, const Atl
 // tap code, looped: the kernel is instruction-fetch bound when it is inlined
 // six times per step).
 __device__ __forceinline__ void sample_clipmap_grad(float4* __restrict__ G, const AtlasDims& A,
-                                                    const vct_cone_tracing_desc& d, float3 p, int level, float3 fo,
+                                                    const MarchScale& C, const vct_cone_tracing_desc& d, float3 p,
+                                                    int level, float3 fo,
                                                     float3 wt, float4 g) {
-    float vs = d.voxel_size * exp2f((float)level);
-    float extent = vs * d.volume_dimension;
-    float dim = d.volume_dimension;
-    float sx = (fractf(p.x / extent) * dim + 1.0f) / (dim + 2.0f);
-    float sy = (fractf(p.y / extent) * dim + 1.0f) / (dim + 2.0f);
-    float sz = (fractf(p.z / extent) * dim + 1.0f) / (dim + 2.0f);
-    sy = sy + (float)level;
-    sy = sy / (float)kClipLevels;
-    sx = sx / (float)kFaces;
+    const float3 s = clipmap_coords(C, d, p, level);
 #pragma unroll 1
     for (int f = 0; f < 3; ++f) {
         const float off = f == 0 ? fo.x : (f == 1 ? fo.y : fo.z);
         const float w = f == 0 ? wt.x : (f == 1 ? wt.y : wt.z);
-        texture3d_grad(G, A, sx + off, sy, sz, make_float4(g.x * w, g.y * w, g.z * w, g.w * w));
+        texture3d_grad(G, A, s.x + off, s.y, s.z, make_float4(g.x * w, g.y * w, g.z * w, g.w * w));
     }
 }
 
 // g(s) of one step spread over its levels, faces and texels.
-__device__ __forceinline__ void scatter_step(float4* __restrict__ G, const AtlasDims& A, const vct_cone_tracing_desc& d,
+__device__ __forceinline__ void scatter_step(float4* __restrict__ G, const AtlasDims& A, const MarchScale& C,
+                                             const vct_cone_tracing_desc& d,
                                              const ConeGeo& K, float3 pos, int lower, int upper, float fr, float4 gs) {
     // s = lo (1 - fr) + hi fr: the lower level's share, then the upper's (zero when fr = 0)
 #pragma unroll 1
     for (int lv = 0; lv < 2; ++lv) {
         const float f = lv ? fr : 1.0f - fr;
         if (f == 0.0f) continue;
-        sample_clipmap_grad(G, A, d, pos, lv ? upper : lower, K.fo, K.wt,
+        sample_clipmap_grad(G, A, C, d, pos, lv ? upper : lower, K.fo, K.wt,
                             make_float4(gs.x * f, gs.y * f, gs.z * f, gs.w * f));
     }
 }
@@ -141,10 +135,11 @@ __device__ __forceinline__ float opacity_slope(const StepDetail& e) {
 
 // One step of trace_cone (same expressions) at march state m: advances m
 // (alpha, occlusion, schedule) and returns the step.
-__device__ __forceinline__ StepDetail march_step(const F4Atlas& T, const vct_cone_tracing_desc& d, const ConeGeo& K,
+__device__ __forceinline__ StepDetail march_step(const F4Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
+                                                 const ConeGeo& K,
                                                  MarchState& m) {
     const Sched s{m.step, m.seg, m.diameter};
-    const StepDetail e = exact_step_detail(T, d, K, s);
+    const StepDetail e = exact_step_detail(T, C, d, K, s);
     const float k = clampf(1.0f - m.alpha, 0.0f, 1.0f);
     m.alpha = m.alpha + k * e.op;
     m.occ = m.occ + (1.0f - m.occ) * e.op / e.q;
@@ -164,7 +159,8 @@ __device__ __forceinline__ StepDetail march_step(const F4Atlas& T, const vct_con
 // segment, kept in local arrays.
 // `rec`: the warp's record block (kRecWarpFloats floats), written and read
 // by each lane for its own cone only.
-__device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, const vct_cone_tracing_desc& d,
+__device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, const MarchScale& C,
+                                   const vct_cone_tracing_desc& d,
                                    const ConeGeo& K, float3 gC, float gO, bool active, float max_dist,
                                    float* rec, int* __restrict__ err) {
     constexpr unsigned kFull = 0xffffffffu;
@@ -182,7 +178,7 @@ __device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, con
         if (running) {
             if ((j % kSegSteps) == 0 && j >= kStoredSteps) ckpt[j / kSegSteps] = m;
             const float alpha0 = m.alpha, occ0 = m.occ, step0 = m.step;
-            const StepDetail e = march_step(T, d, K, m);
+            const StepDetail e = march_step(T, C, d, K, m);
             if (j < kStoredSteps) {
                 float* r = rec + (size_t)j * 32 + lane;
                 constexpr size_t F = (size_t)kStoredSteps * 32;  // one field's floats
@@ -232,7 +228,7 @@ __device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, con
                 if (k_raw >= 0.0f && k_raw <= 1.0f) gA = gA - ((gC.x * sr + gC.y * sg + gC.z * sb) * c + gA * op);
                 gO = gO * (1.0f - op / q);
                 const float3 pos = K.start + K.dir * step;  // exact_step_detail's expression
-                scatter_step(G, T.A, d, K, pos, (int)(short)(lv & 0xffff), lv >> 16, fr, gs);
+                scatter_step(G, T.A, C, d, K, pos, (int)(short)(lv & 0xffff), lv >> 16, fr, gs);
             }
             continue;
         }
@@ -241,7 +237,7 @@ __device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, con
         for (int i = first; i < last; ++i) {
             if (i < mine) {
                 seg[i - first] = r;
-                seg_step[i - first] = march_step(T, d, K, r);
+                seg_step[i - first] = march_step(T, C, d, K, r);
             }
         }
         for (int i = last - 1; i >= first; --i) {
@@ -260,7 +256,7 @@ __device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, con
             if (k_raw >= 0.0f && k_raw <= 1.0f)
                 gA = gA - ((gC.x * e.smp.x + gC.y * e.smp.y + gC.z * e.smp.z) * c + gA * e.op);
             gO = gO * (1.0f - e.op / e.q);
-            scatter_step(G, T.A, d, K, e.pos, e.lower, e.upper, e.fr, gs);
+            scatter_step(G, T.A, C, d, K, e.pos, e.lower, e.upper, e.fr, gs);
         }
     }
 }
@@ -290,7 +286,8 @@ __device__ __forceinline__ bool diffuse_seeds(const TraceParams& P, const GSampl
     return !(gC.x == 0.0f && gC.y == 0.0f && gC.z == 0.0f && gO == 0.0f);
 }
 
-__global__ void __launch_bounds__(128) k_cone_backward_diffuse(TraceParams P, F4Atlas T,
+__global__ void __launch_bounds__(128) k_cone_backward_diffuse(const __grid_constant__ TraceParams P,
+                                                               const __grid_constant__ MarchScale C, F4Atlas T,
                                                                const vct_surface_sample* __restrict__ samples,
                                                                int64_t n, const uint32_t* __restrict__ order,
                                                                const float4* __restrict__ gd, float4* __restrict__ G,
@@ -333,16 +330,17 @@ __global__ void __launch_bounds__(128) k_cone_backward_diffuse(TraceParams P, F4
         float3 gC = f3(0.f, 0.f, 0.f);
         float gO = 0.0f;
         active = active && diffuse_seeds(P, g, gd[i], cos_t, nc, gC, gO);
-        const ConeGeo K = make_cone(d, start, dir, P.diffuse_aperture, min_level,
+        const ConeGeo K = make_cone(d, start, dir, cone_coef(P.diffuse_aperture), min_level,
                                     fmaxf(kMinTraceStepFactor, d.min_trace_step_factor));
-        cone_backward_lane(T, G, d, K, gC, gO, active, kMaxTraceDistance, rec, err);
+        cone_backward_lane(T, G, C, d, K, gC, gO, active, kMaxTraceDistance, rec, err);
     }
 }
 
 // One lane per specular cone of the aperture-grouped list (a warp's cones
 // share their step schedule, so the lock-step walk keeps its lanes busy).
 __global__ void __launch_bounds__(128) k_cone_backward_specular(
-    TraceParams P, F4Atlas T, const vct_surface_sample* __restrict__ samples, const uint32_t* __restrict__ list,
+    const __grid_constant__ TraceParams P, const __grid_constant__ MarchScale C, F4Atlas T,
+    const vct_surface_sample* __restrict__ samples, const uint32_t* __restrict__ list,
     const unsigned int* __restrict__ spec_count, const float4* __restrict__ gsp, float4* __restrict__ G,
     float* rec_all, int* __restrict__ err) {
     const vct_cone_tracing_desc& d = P.d;
@@ -366,8 +364,9 @@ __global__ void __launch_bounds__(128) k_cone_backward_specular(
         const float vs = d.voxel_size * exp2f(min_level);
         const float3 start = g.wp + g.normal * (vs * d.trace_start_offset);
         const float3 sdir = reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal);
-        const ConeGeo K = make_cone(d, start, sdir, fmaxf(g.roughness, kMinSpecularAperture), min_level, d.voxel_size);
-        cone_backward_lane(T, G, d, K, gC, 0.0f, active, kMaxTraceDistance, rec, err);
+        const ConeGeo K = make_cone(d, start, sdir, cone_coef(fmaxf(g.roughness, kMinSpecularAperture)), min_level,
+                                    d.voxel_size);
+        cone_backward_lane(T, G, C, d, K, gC, 0.0f, active, kMaxTraceDistance, rec, err);
     }
 }
 
@@ -414,6 +413,7 @@ extern "C" int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const 
         return fail(VCT_E_CUDA, "vct_cone_trace_backward: record scratch allocation failed");
     }
     F4Atlas T{reinterpret_cast<const float4*>(atlas4), AtlasDims(R)};
+    const MarchScale C = march_scale(P.d);
     ExactPlan plan;
     rc = exact_plan(samples, n, P.d, &plan, st);
     if (rc != VCT_OK) {
@@ -422,11 +422,11 @@ extern "C" int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const 
         return rc;
     }
     float4* G = reinterpret_cast<float4*>(grad_atlas4);
-    k_cone_backward_diffuse<<<(int)blocks, 128, 0, st>>>(P, T, samples, n, plan.order,
+    k_cone_backward_diffuse<<<(int)blocks, 128, 0, st>>>(P, C, T, samples, n, plan.order,
                                                           reinterpret_cast<const float4*>(grad_diffuse), G, rec, err);
     cudaError_t le = cudaGetLastError();
     if (le == cudaSuccess) {
-        k_cone_backward_specular<<<(int)lblocks, 128, 0, st>>>(P, T, samples, plan.spec_list, plan.spec_count,
+        k_cone_backward_specular<<<(int)lblocks, 128, 0, st>>>(P, C, T, samples, plan.spec_list, plan.spec_count,
                                                                reinterpret_cast<const float4*>(grad_specular), G, rec,
                                                                err);
         le = cudaGetLastError();
