@@ -102,3 +102,31 @@ def test_dense_pool_against_the_oracle(cuda, oracle, dim, voxel, box, over):
         # cell border may then take its neighbour)
         assert np.mean(err < 1e-4) > 0.99, np.sort(err)[-8:]
     assert abs(int(steps.item()) - st32) <= max(8, 0.002 * st32)
+
+
+@pytest.mark.gpu
+def test_octree_cone_groups_march_alike(cuda):
+    """The octree trace of 300 specular samples, alone (8 lanes a cone) and repeated until fewer march one."""
+    torch = cuda
+    from vk_voxel_cone_tracing_gb300 import clipmap, passes
+    from vk_voxel_cone_tracing_gb300.scene import random_samples
+    pool = torch.from_numpy(dense_pool(5, 3).view(np.int32).copy()).cuda()
+    desc = clipmap.trace_desc(volume_center=[0.0, 0.0, 0.0], rendering_mode=8, voxel_size=0.25, volume_dimension=32.0,
+                              trace_start_offset=1.0, indirect_diffuse_intensity=8.0, ambient_occlusion_factor=0.5,
+                              min_trace_step_factor=1.0, indirect_specular_intensity=3.0, occlusion_decay=0.05,
+                              enable_32_cones=0)
+    box = dict(bb_min=(-4.0, -4.0, -4.0), bb_max=(4.0, 4.0, 4.0))
+
+    def run(s):
+        steps = torch.zeros(1, dtype=torch.int64, device="cuda")
+        d, sp = passes.svo_cone_trace(desc, (0.0, 1.0, -4.0), pool, pool.shape[0], s, steps=steps, **box)
+        return d, sp, int(steps.item())
+
+    probe = clipmap.samples_to_device(random_samples(3000, (0, 0, 0), 3.0, seed=6))
+    few = probe[run(probe)[1][:, :3].abs().sum(1) > 0][:300].contiguous()
+    assert few.shape[0] == 300
+    d, sp, steps = run(few)
+    for times in (150, 400, 1100):  # 45,000 to 330,000 cones for 311,296 lanes
+        D, S, n = run(few.repeat(times, 1))
+        assert torch.equal(torch.nan_to_num(D), torch.nan_to_num(d.repeat(times, 1)))
+        assert torch.equal(S, sp.repeat(times, 1)) and n == steps * times

@@ -25,8 +25,8 @@
 //   * a step whose two nodes are zero leaves the composite as it is, so level
 //     size, opacity power and divisions run for the others alone.
 // Measured: the trace of 1,000,003 samples on the 4M-triangle terrain at
-// L = 9 went from 4.9 to 1.4 ms, 65,536 samples on the room at L = 7 from 0.57
-// to 0.42 ms, every output unchanged.
+// L = 9 went from 4.9 to 1.3 ms, 65,536 samples on the room at L = 7 from 0.57
+// to 0.17 ms, every output unchanged.
 #include <cmath>
 
 #include "trace_deal.cuh"
@@ -95,48 +95,42 @@ __device__ __forceinline__ float svo_over_uvs(const SvoScene& S, float x, float 
     return S.uvs_pow2 ? x * S.inv_uvs : x / uvs;
 }
 
-// traceCone over the pool.  level_at[k] (k < levels): log2(diameter / uvs) of step k, where the caller has it.
-__device__ float4 svo_trace_cone(const SvoScene& S, const vct_cone_tracing_desc& d, float3 start, float3 dir,
-                                 float cone_coef, float start_level, float step_factor, const float* level_at,
-                                 int levels, unsigned long long& steps) {
-    float4 result = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float uvs = d.voxel_size;
-    float vs = uvs * exp2f(start_level);
-    start = start + dir * (vs * d.trace_start_offset * 0.5f);
-    float step = 0.0f, diameter = fmaxf(step * cone_coef, uvs), occlusion = 0.0f, seg = vs;
-    const float3 center = f3(d.volume_center[0], d.volume_center[1], d.volume_center[2]);
+// One step of traceCone over the pool.
+__device__ __forceinline__ StepTerm svo_step(const SvoScene& S, const vct_cone_tracing_desc& d, const ConeGeo& K,
+                                             float step, float seg, float raw_level) {
+    const float3 pos = K.start + K.dir * step;
+    const float min_level = cone_min_level(S.inv_r2, S.min_radius, K.center, pos);
+    const float level = fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
+    const uint2 v = svo_nodes(S, pos, (uint32_t)floorf(level), (uint32_t)ceilf(level));
+    StepTerm t;
+    t.some = (v.x | v.y) != 0u;
+    if (!t.some) return t;
+    const float4 a = unpack_rgba8(v.x), b = unpack_rgba8(v.y);
+    const float fr = fractf(level);
+    return cone_term(d, K, step, seg, level,
+                     make_float4(a.x * (1.0f - fr) + b.x * fr, a.y * (1.0f - fr) + b.y * fr,
+                                 a.z * (1.0f - fr) + b.z * fr, a.w * (1.0f - fr) + b.w * fr));
+}
+
+__device__ __forceinline__ float4 svo_result(const ConeSum& sum) {
+    const float4 r = sum.result();
+    return make_float4(clampf(r.x, 0.f, 1.f), clampf(r.y, 0.f, 1.f), clampf(r.z, 0.f, 1.f), clampf(r.w, 0.f, 1.f));
+}
+
+// traceCone on one lane.  level_at[k] (k < levels): log2(diameter / uvs) of step k, where the caller has it.
+__device__ float4 svo_trace_cone(const SvoScene& S, const vct_cone_tracing_desc& d, const ConeGeo& K,
+                                 const float* level_at, int levels, unsigned long long& steps) {
+    ConeSum sum{make_float4(0.f, 0.f, 0.f, 0.f), 0.0f};
+    Sched s = first_sched(K);
     int k = 0;
-    while (step < kMaxTraceDistance && occlusion < 1.0f) {
-        const float3 pos = start + dir * step;
-        const float min_level = cone_min_level(S.inv_r2, S.min_radius, center, pos);
-        float cur_level;
-        if (k < levels) cur_level = level_at[k];
-        else cur_level = log2f(svo_over_uvs(S, diameter, uvs));
-        ++k;
-        cur_level = fminf(fmaxf(fmaxf(start_level, cur_level), min_level), (float)(kClipLevels - 1));
-        const uint2 v = svo_nodes(S, pos, (uint32_t)floorf(cur_level), (uint32_t)ceilf(cur_level));
-        if (v.x | v.y) {
-            const float4 a = unpack_rgba8(v.x), b = unpack_rgba8(v.y);
-            const float fr = fractf(cur_level);
-            const float4 s = make_float4(a.x * (1.0f - fr) + b.x * fr, a.y * (1.0f - fr) + b.y * fr,
-                                         a.z * (1.0f - fr) + b.z * fr, a.w * (1.0f - fr) + b.w * fr);
-            vs = uvs * exp2f(cur_level);
-            const float correction = seg / vs;
-            const float rx = s.x * correction, ry = s.y * correction, rz = s.z * correction;
-            // alpha rounded above 1 (a pow of a negative base, undefined in GLSL) is taken as 1
-            const float opacity = clampf(1.0f - powf(fmaxf(1.0f - s.w, 0.0f), correction), 0.0f, 1.0f);
-            const float q = clampf(1.0f - result.w, 0.0f, 1.0f);
-            result = make_float4(result.x + q * rx, result.y + q * ry, result.z + q * rz, result.w + q * opacity);
-            occlusion = occlusion + (1.0f - occlusion) * opacity / (1.0f + (step + vs) * d.occlusion_decay);
-        }
-        const float prev = step;
-        step = step + fmaxf(diameter, uvs) * step_factor;
-        seg = step - prev;
-        diameter = step * cone_coef;
+    for (; s.step < kMaxTraceDistance && sum.occlusion < 1.0f; ++k) {
+        const float raw = k < levels ? level_at[k] : log2f(svo_over_uvs(S, s.diameter, K.uvs));
+        const StepTerm t = svo_step(S, d, K, s.step, s.seg, raw);
+        if (t.some) sum.add(t.c, t.op, t.q);
+        sched_advance(s, K);
     }
     steps += (unsigned)k;
-    return make_float4(clampf(result.x, 0.f, 1.f), clampf(result.y, 0.f, 1.f), clampf(result.z, 0.f, 1.f),
-                       clampf(1.0f - occlusion, 0.f, 1.f));
+    return svo_result(sum);
 }
 
 // The rendering-mode switch of voxelConeTracing_Octree.frag, its two outputs.
@@ -206,6 +200,9 @@ struct SvoFinish {
 
 constexpr int kSvoWarps = 4;  // warps per block of the diffuse kernel
 constexpr int kSvoWarpsPerSm = 16;  // warp items per SM that deal_samples_per_warp aims at
+// Warps per SM of a full specular grid, which the lanes per cone follow
+// (65,536 samples on the room, us of the whole case: 16: 954, 32: 894, 40: 893, 64: 872).
+constexpr int kSvoSpecWarpsPerSm = 64;
 constexpr int kSvoLevels = 128;  // steps of the diffuse schedule kept as a table (default descriptors take 19 to 40)
 
 struct SvoDiffuseMarch {
@@ -216,7 +213,7 @@ struct SvoDiffuseMarch {
     int levels;
     __device__ __forceinline__ float4 operator()(float3 start, float3 dir, float start_level,
                                                  unsigned long long& steps) const {
-        return svo_trace_cone(*S, *d, start, dir, coef, start_level, step_factor, level_at, levels, steps);
+        return svo_trace_cone(*S, *d, make_cone(*d, start, dir, coef, start_level, step_factor), level_at, levels, steps);
     }
 };
 
@@ -253,8 +250,8 @@ __global__ void __launch_bounds__(32 * kSvoWarps) k_svo_diffuse(const __grid_con
     add_steps(step_counter, steps);
 }
 
-// One lane per specular cone of the aperture-grouped list, 32 at a time to
-// the warps as they free up.
+// A group of lanes (cone_group) per specular cone of the aperture-grouped
+// list, a warp's worth at a time to the warps as they free up.
 __global__ void __launch_bounds__(128) k_svo_specular(const __grid_constant__ TraceParams P,
                                                       const __grid_constant__ SvoScene S,
                                                       const vct_surface_sample* __restrict__ samples,
@@ -266,23 +263,36 @@ __global__ void __launch_bounds__(128) k_svo_specular(const __grid_constant__ Tr
     const vct_cone_tracing_desc& d = P.d;
     const uint32_t m = *spec_count;
     const int lane = threadIdx.x & 31;
+    const int group = cone_group(m), cones = 32 / group, first = lane & ~(group - 1);
     unsigned long long steps = 0;
     for (;;) {
         uint32_t c0 = 0;
-        if (lane == 0) c0 = atomicAdd(ticket, 32u);
+        if (lane == 0) c0 = atomicAdd(ticket, (unsigned)cones);
         c0 = __shfl_sync(0xffffffffu, c0, 0);
         if (c0 >= m) break;
-        const uint32_t c = c0 + (uint32_t)lane;
-        if (c >= m) continue;
-        const uint32_t idx = __ldg(list + c);
+        const uint32_t c = c0 + (uint32_t)(lane / group);
+        const bool valid = c < m;
+        const uint32_t idx = __ldg(list + (valid ? c : c0));
         const GSample g = load_sample(samples + idx, P.eye);
         const float min_level = calc_min_level(d, g.wp);
         const float vs = d.voxel_size * exp2f(min_level);
         const float3 start = g.wp + g.normal * (vs * d.trace_start_offset);
         const float3 sdir = normalize3(reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal));
-        const float coef = 2.0f * tanf(fmaxf(g.roughness, kMinSpecularAperture) * 0.5f);
-        const float4 r = svo_trace_cone(S, d, start, sdir, coef, min_level, fmaxf(kMinTraceStepFactor, d.voxel_size),
-                                        nullptr, 0, steps);
+        const ConeGeo K = make_cone(d, start, sdir, cone_coef(fmaxf(g.roughness, kMinSpecularAperture)), min_level,
+                                    fmaxf(kMinTraceStepFactor, d.voxel_size));
+        float4 r;
+        if (group == 1) {  // the groups' ballots and shuffles cost a tenth of a long list's time
+            if (!valid) continue;
+            r = svo_trace_cone(S, d, K, nullptr, 0, steps);
+        } else {
+            unsigned int taken = 0;
+            const ConeSum sum = march_group(K, group, valid, [&](const Sched& s) {
+                return svo_step(S, d, K, s.step, s.seg, log2f(svo_over_uvs(S, s.diameter, K.uvs)));
+            }, taken);
+            if (lane != first || !valid) continue;
+            steps += taken;
+            r = svo_result(sum);
+        }
         const float isi = d.indirect_specular_intensity;
         reinterpret_cast<float4*>(sout)[idx] = svo_specular_out(
             d.rendering_mode,
@@ -354,8 +364,8 @@ extern "C" int vct_svo_cone_trace(const vct_cone_tracing_desc* desc, const vct_c
             P, S, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, plan.spec_count + 2, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            const int64_t gs = (m + 127) / 128;
-            k_svo_specular<<<(int)(gs > 152 * 8 ? 152 * 8 : gs), 128, 0, st>>>(
+            const int64_t gs = (m * kMaxConeGroup + 127) / 128, full = 152 * kSvoSpecWarpsPerSm / 4;
+            k_svo_specular<<<(int)(gs > full ? full : gs), 128, 0, st>>>(
                 P, S, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, plan.spec_count + 1);
             e = cudaGetLastError();
         }

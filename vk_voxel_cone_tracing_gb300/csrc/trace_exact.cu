@@ -86,21 +86,13 @@ __global__ void __launch_bounds__(32 * kExactWarps) k_exact_diffuse(const __grid
     add_steps(step_counter, steps);
 }
 
-// Lanes per specular cone: a power of two up to kExactMaxGroup, as few as give
-// kExactSpecWarpsPerSm warps per SM.  Measured (whole trace, 65,536 cones, us):
-// two lanes 1,485, four 1,145, eight 1,154; every further lane repeats the
-// additions, so larger lists take fewer.
-constexpr int kExactMaxGroup = 8;
-constexpr int kExactSpecWarpsPerSm = 32;
+constexpr int kExactSpecWarpsPerSm = 32;  // warps per SM of a full specular grid
 
-// One group of `group` lanes per specular cone of the list.  The list is
+// A group of lanes (cone_group) per specular cone of the list.  The list is
 // grouped by aperture (then kept in the coherent order), and a cone's step
 // count depends only on its aperture (and the occlusion stop), so a warp's
-// cones march in step; 32 / group consecutive cones go to a warp at a time as
-// warps free up, the longest first.  The group's lanes take consecutive steps:
-// each samples its own, then all add the terms in step order, so every cone's
-// sum is the one-lane march's bit for bit (the steps after the occlusion stop
-// are dropped).
+// cones march in step; as many consecutive cones as a warp has groups go to it
+// at a time as warps free up, the longest first.
 template <class Atlas>
 __global__ void __launch_bounds__(128) k_exact_specular(const __grid_constant__ TraceParams P,
                                                         const __grid_constant__ MarchScale C,
@@ -115,10 +107,7 @@ __global__ void __launch_bounds__(128) k_exact_specular(const __grid_constant__ 
     const vct_cone_tracing_desc& d = P.d;
     const int64_t m = *spec_count;
     const int lane = threadIdx.x & 31;
-    int group = 1;
-    while (group < kExactMaxGroup && m * group < (int64_t)gridDim.x * 128) group <<= 1;
-    const int cones = 32 / group, first = lane & ~(group - 1);
-    const uint32_t firsts = group == 1 ? kFull : (group == 2 ? 0x55555555u : (group == 4 ? 0x11111111u : 0x01010101u));
+    const int group = cone_group(m), cones = 32 / group, first = lane & ~(group - 1);
     unsigned long long steps = 0;
     for (;;) {
         uint32_t c0 = 0;
@@ -135,38 +124,10 @@ __global__ void __launch_bounds__(128) k_exact_specular(const __grid_constant__ 
         const float3 sdir = reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal);
         const ConeGeo K = make_cone(d, start, sdir, cone_coef(fmaxf(g.roughness, kMinSpecularAperture)), min_level,
                                     d.voxel_size);
-        ConeSum sum{make_float4(0.f, 0.f, 0.f, 0.f), 0.0f};
-        Sched s = first_sched(K);  // the group's next unsampled step, the same on its lanes
-        bool running = valid && s.step < kMaxTraceDistance;
         unsigned int taken = 0;
-        while (__any_sync(kFull, running)) {
-            Sched mine = s;
-            for (int j = 0; j < group; ++j) {
-                if (lane - first == j) mine = s;
-                sched_advance(s, K);
-            }
-            const bool has = running && mine.step < kMaxTraceDistance;
-            StepTerm t;
-            t.some = false;
-            if (has)
-                t = exact_step(T, C, d, K, mine.step, mine.seg, cone_raw_level(C, mine.diameter, K.uvs));
-            const uint32_t has_mask = __ballot_sync(kFull, has) >> first, some = __ballot_sync(kFull, t.some);
-            if (some == 0u) {  // nothing to add in the warp
-                taken += __popc(has_mask & ((2u << (group - 1)) - 1u));
-            } else {
-                for (int j = 0; j < group; ++j) {
-                    const bool on = ((has_mask >> j) & 1u) && sum.occlusion < 1.0f;
-                    taken += on;
-                    if (!((some >> j) & firsts)) continue;  // no cone of the warp adds at its step j
-                    const int src = first + j;
-                    const float3 rc = f3(__shfl_sync(kFull, t.c.x, src), __shfl_sync(kFull, t.c.y, src),
-                                         __shfl_sync(kFull, t.c.z, src));
-                    const float op = __shfl_sync(kFull, t.op, src), q = __shfl_sync(kFull, t.q, src);
-                    if (on && ((some >> src) & 1u)) sum.add(rc, op, q);
-                }
-            }
-            running = running && s.step < kMaxTraceDistance && sum.occlusion < 1.0f;
-        }
+        const ConeSum sum = march_group(K, group, valid, [&](const Sched& s) {
+            return exact_step(T, C, d, K, s.step, s.seg, cone_raw_level(C, s.diameter, K.uvs));
+        }, taken);
         if (lane != first || !valid) continue;
         steps += taken;
         const float4 r = sum.result();
@@ -414,7 +375,7 @@ static int launch_exact(const TraceParams& P, const Atlas& T, const vct_surface_
             P, C, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            const int64_t gl = (m * kExactMaxGroup + 127) / 128, full = 152 * kExactSpecWarpsPerSm / 4;
+            const int64_t gl = (m * kMaxConeGroup + 127) / 128, full = 152 * kExactSpecWarpsPerSm / 4;
             k_exact_specular<<<(int)(gl > full ? full : gl), 128, 0, st>>>(
                 P, C, T, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, spec_ticket);
             e = cudaGetLastError();

@@ -320,18 +320,12 @@ struct StepTerm {
     bool some;  // false: all of it leaves the composite as it is
 };
 
-// One step of traceCone's loop (voxelConeTracing.frag:341-392) up to the
-// composite.  `raw_level`: cone_raw_level of the step's diameter.
-template <class Atlas>
-__device__ __forceinline__ StepTerm exact_step(const Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
-                                               const ConeGeo& K, float step, float seg, float raw_level) {
-    const float3 pos = K.start + K.dir * step;
-    const float min_level = cone_min_level(C.inv_r2, C.min_radius, K.center, pos);
-    const float level = fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
-    const float4 s = sample_levels(T, C, d, pos, level, K.fo, K.wt);
+// traceCone's loop (voxelConeTracing.frag:341-392) from the sample s of one
+// step, at `level`, to the composite.
+__device__ __forceinline__ StepTerm cone_term(const vct_cone_tracing_desc& d, const ConeGeo& K, float step, float seg,
+                                              float level, float4 s) {
     StepTerm t;
-    t.some = s.x != 0.0f || s.y != 0.0f || s.z != 0.0f || s.w != 0.0f || !(d.occlusion_decay >= 0.0f);
-    if (!t.some) return t;
+    t.some = true;
     const float vs = K.uvs * exp2f(level);
     const float correction = seg / vs;
     t.c = f3(s.x * correction, s.y * correction, s.z * correction);
@@ -341,6 +335,19 @@ __device__ __forceinline__ StepTerm exact_step(const Atlas& T, const MarchScale&
     t.op = clampf(1.0f - powf(fmaxf(1.0f - s.w, 0.0f), correction), 0.0f, 1.0f);
     t.q = 1.0f + (step + vs) * d.occlusion_decay;
     return t;
+}
+
+// One step over a clipmap atlas.  `raw_level`: cone_raw_level of the step's diameter.
+template <class Atlas>
+__device__ __forceinline__ StepTerm exact_step(const Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
+                                               const ConeGeo& K, float step, float seg, float raw_level) {
+    const float3 pos = K.start + K.dir * step;
+    const float min_level = cone_min_level(C.inv_r2, C.min_radius, K.center, pos);
+    const float level = fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
+    const float4 s = sample_levels(T, C, d, pos, level, K.fo, K.wt);
+    StepTerm t;
+    t.some = s.x != 0.0f || s.y != 0.0f || s.z != 0.0f || s.w != 0.0f || !(d.occlusion_decay >= 0.0f);
+    return t.some ? cone_term(d, K, step, seg, level, s) : t;
 }
 
 struct ConeSum {
@@ -371,6 +378,63 @@ __device__ __forceinline__ float4 trace_cone(const Atlas& T, const MarchScale& C
     }
     steps += (unsigned)k;
     return sum.result();
+}
+
+// traceCone by `group` lanes (a power of two up to 8; the whole warp calls,
+// 32 / group cones side by side): the lanes of a group take consecutive steps,
+// each samples its own (`at(sched)`, a StepTerm), then all add the terms in
+// step order, so the sum is the one-lane march's bit for bit and the steps
+// after the occlusion stop are dropped.  Every lane returns its cone's sum and
+// adds the cone's steps to `taken`.
+template <class StepFn>
+__device__ __forceinline__ ConeSum march_group(const ConeGeo& K, int group, bool valid, const StepFn& at,
+                                               unsigned int& taken) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, first = lane & ~(group - 1);
+    const uint32_t firsts = group == 1 ? kFull : (group == 2 ? 0x55555555u : (group == 4 ? 0x11111111u : 0x01010101u));
+    ConeSum sum{make_float4(0.f, 0.f, 0.f, 0.f), 0.0f};
+    Sched s = first_sched(K);  // the group's next step, the same on its lanes
+    bool running = valid && s.step < kMaxTraceDistance;
+    while (__any_sync(kFull, running)) {
+        Sched mine = s;
+        for (int j = 0; j < group; ++j) {
+            if (lane - first == j) mine = s;
+            sched_advance(s, K);
+        }
+        const bool has = running && mine.step < kMaxTraceDistance;
+        StepTerm t;
+        t.some = false;
+        if (has) t = at(mine);
+        const uint32_t has_mask = __ballot_sync(kFull, has) >> first, some = __ballot_sync(kFull, t.some);
+        if (some == 0u) {  // nothing to add in the warp
+            taken += __popc(has_mask & ((2u << (group - 1)) - 1u));
+        } else {
+            for (int j = 0; j < group; ++j) {
+                const bool on = ((has_mask >> j) & 1u) && sum.occlusion < 1.0f;
+                taken += on;
+                if (!((some >> j) & firsts)) continue;  // no cone of the warp adds at its step j
+                const int src = first + j;
+                const float3 rc = f3(__shfl_sync(kFull, t.c.x, src), __shfl_sync(kFull, t.c.y, src),
+                                     __shfl_sync(kFull, t.c.z, src));
+                const float op = __shfl_sync(kFull, t.op, src), q = __shfl_sync(kFull, t.q, src);
+                if (on && ((some >> src) & 1u)) sum.add(rc, op, q);
+            }
+        }
+        running = running && s.step < kMaxTraceDistance && sum.occlusion < 1.0f;
+    }
+    return sum;
+}
+
+// Lanes per specular cone of a list of m: a power of two up to kMaxConeGroup,
+// as few as give every lane of the grid work.  Measured (whole exact trace,
+// 65,536 cones on a grid of 32 warps per SM, us): two lanes 1,485, four 1,145,
+// eight 1,154; every further lane repeats the additions, so larger lists take
+// fewer.
+constexpr int kMaxConeGroup = 8;
+__device__ __forceinline__ int cone_group(int64_t m) {
+    int group = 1;
+    while (group < kMaxConeGroup && m * group < (int64_t)gridDim.x * blockDim.x) group <<= 1;
+    return group;
 }
 
 // Everything one step computes: its tap geometry (position, the two levels
