@@ -56,8 +56,8 @@ __device__ __forceinline__ uint2 to_h4(uint32_t v) {
 // since a 32-byte sector of the array's block-linear layout holds two texels
 // of two neighbouring rows: every sector a warp writes is written whole
 // (row-by-row warps wrote half sectors and paid a read-modify-write for each).
-// Bound by the writes (12 bytes read and written a byte of texel with the
-// array): one texel a thread, one slice at a time took 357 us at R = 128;
+// Bound by its bytes (4 read and 16 written a texel, the array's included):
+// one texel a thread, one slice at a time took 357 us at R = 128;
 // this, 239 (four or eight slices: the same).
 // PAIRS: src and dst at pairs' alignment (8 and 16 bytes; W is even), moved
 // in one access; without, texel by texel.

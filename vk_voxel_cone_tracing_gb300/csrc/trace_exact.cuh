@@ -337,13 +337,21 @@ __device__ __forceinline__ StepTerm cone_term(const vct_cone_tracing_desc& d, co
     return t;
 }
 
+// The step's level (raw_level: cone_raw_level of its diameter).
+__device__ __forceinline__ float clamp_level(const MarchScale& C, const ConeGeo& K, float3 pos, float raw_level) {
+    const float min_level = cone_min_level(C.inv_r2, C.min_radius, K.center, pos);
+    return fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
+}
+__device__ __forceinline__ float step_level(const MarchScale& C, const ConeGeo& K, float3 pos, float diameter) {
+    return clamp_level(C, K, pos, cone_raw_level(C, diameter, K.uvs));
+}
+
 // One step over a clipmap atlas.  `raw_level`: cone_raw_level of the step's diameter.
 template <class Atlas>
 __device__ __forceinline__ StepTerm exact_step(const Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
                                                const ConeGeo& K, float step, float seg, float raw_level) {
     const float3 pos = K.start + K.dir * step;
-    const float min_level = cone_min_level(C.inv_r2, C.min_radius, K.center, pos);
-    const float level = fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
+    const float level = clamp_level(C, K, pos, raw_level);
     const float4 s = sample_levels(T, C, d, pos, level, K.fo, K.wt);
     StepTerm t;
     t.some = s.x != 0.0f || s.y != 0.0f || s.z != 0.0f || s.w != 0.0f || !(d.occlusion_decay >= 0.0f);
@@ -437,13 +445,10 @@ __device__ __forceinline__ int cone_group(int64_t m) {
     return group;
 }
 
-// Everything one step computes: its tap geometry (position, the two levels
-// and the mix fraction), the filtered sample, the opacity correction, the raw
-// and clamped opacity and the occlusion divisor.
+// What one step computes for the adjoint: the filtered sample, the opacity
+// correction, the raw and clamped opacity and the occlusion divisor.
 struct StepDetail {
-    float3 pos;
-    int lower, upper;
-    float fr, correction, op_raw, op, q;
+    float correction, op_raw, op, q;
     float4 smp;
 };
 
@@ -452,17 +457,12 @@ __device__ __forceinline__ StepDetail exact_step_detail(const Atlas& T, const Ma
                                                         const vct_cone_tracing_desc& d, const ConeGeo& K,
                                                         const Sched& s) {
     StepDetail e;
-    e.pos = K.start + K.dir * s.step;
-    const float min_level = cone_min_level(C.inv_r2, C.min_radius, K.center, e.pos);
-    const float level = cone_raw_level(C, s.diameter, K.uvs);
-    const float cur_level = fminf(fmaxf(fmaxf(K.start_level, level), min_level), (float)(kClipLevels - 1));
-    e.lower = (int)floorf(cur_level);
-    e.upper = (int)ceilf(cur_level);
-    e.fr = fractf(cur_level);
-    e.smp = sample_levels(T, C, d, e.pos, cur_level, K.fo, K.wt);
-    const float vs = K.uvs * exp2f(cur_level);
+    const float3 pos = K.start + K.dir * s.step;
+    const float level = step_level(C, K, pos, s.diameter);
+    e.smp = sample_levels(T, C, d, pos, level, K.fo, K.wt);
+    const float vs = K.uvs * exp2f(level);
     e.correction = s.seg / vs;
-    e.op_raw = 1.0f - powf(fmaxf(1.0f - e.smp.w, 0.0f), e.correction);  // base >= 0 as in exact_step
+    e.op_raw = 1.0f - powf(fmaxf(1.0f - e.smp.w, 0.0f), e.correction);  // base >= 0 as in cone_term
     e.op = clampf(e.op_raw, 0.0f, 1.0f);
     e.q = 1.0f + (s.step + vs) * d.occlusion_decay;
     return e;

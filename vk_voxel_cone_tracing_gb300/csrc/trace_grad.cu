@@ -25,14 +25,25 @@
 // Same FP32 expressions as the forward kernels (this unit is built with
 // -fmad=false like them), so the recomputed steps are the forward's.
 //
-// Each cone is walked by one lane, the warp's lanes in lock step: one march
-// forward keeps each of the first 128 steps' record (the state before the
-// step, its sample, opacity terms, position and levels) in device scratch,
-// and a checkpoint of the march state every 32 steps after those; the walk
-// backward with the recurrences above in sequential form reads the records,
-// and recomputes a later segment from its checkpoint.  Diffuse cones all share one step schedule; specular
-// cones are taken from the exact forward's aperture-grouped list, so a
-// warp's cones also march nearly the same number of steps.
+// A cone is walked by one lane or, where the cones are few, by a group of
+// lanes that take consecutive steps (march_group's split): a march forward
+// keeps a record of each of the first kStoredRounds rounds' steps (the state
+// before the step, its opacity terms, its colour against gC, its distance) in
+// device scratch and a checkpoint of the march every kSegRounds rounds after
+// those; the walk backward, with the recurrences above in sequential form,
+// reads the records, a later segment's after marching it again from its
+// checkpoint.  Diffuse cones all share one step schedule; specular cones are
+// taken from the exact forward's aperture-grouped list, so a warp's cones also
+// march nearly the same number of steps.  Work goes to the warps as they free
+// up.
+//
+// Bound by the scatter: up to 48 float4 atomics a step (274 M sectors of them
+// in the diffuse kernel of 65,536 samples at R = 64; L1 wavefronts 61 % and L2
+// 50 % of their peaks).  One lane a cone, 128 steps of 12 fields and a static
+// deal took 1.78 ms for the specular cones, whose longest marches outlast the
+// rest by half, and 1.64 ms for the diffuse ones, with 478 MB of records whose
+// allocation cost another 1.2 ms a call; this takes 1.33 and 1.50 ms with
+// 174 MB.
 #include <algorithm>
 
 #include "trace_exact.cuh"
@@ -45,21 +56,23 @@ int fill_trace_params(TraceParams& P, const vct_cone_tracing_desc* desc, const v
 
 namespace {
 
-constexpr int kSegSteps = 32;
-constexpr int kMaxSegments = 256;  // 8192 steps per cone: the specular cone at R = 1024 takes ~7.1k
+constexpr int kMaxSteps = 8192;  // per cone: the specular cone at R = 1024 takes ~7.1k
+// Rounds (one step a lane) whose records the forward march keeps, and of a
+// segment marched again: default diffuse cones take 19 to 40.
+constexpr int kStoredRounds = 48, kSegRounds = 32;
+constexpr int kMaxSegments = (kMaxSteps - kStoredRounds + kSegRounds - 1) / kSegRounds;
 
-// A cone's first kStoredSteps steps keep what the reverse walk reads in a
-// record block of the lane's warp (device scratch, one block per warp of the
-// grid, fields outermost and lanes innermost: a warp's store or load of a
-// field is one 128-byte line), so those segments are walked backward without
-// a second march; later segments are recomputed from checkpoints.
-constexpr int kStoredSteps = 128;
-static_assert(kStoredSteps % kSegSteps == 0, "stored steps are whole segments");
-enum RecField { kRecAlpha, kRecOcc, kRecCorr, kRecQ, kRecOp, kRecSlope, kRecR, kRecG, kRecB, kRecStep, kRecFr,
-                kRecLevels, kRecFields };
-constexpr size_t kRecWarpFloats = (size_t)kRecFields * kStoredSteps * 32;
-__device__ __forceinline__ void rec_put(float* p, float v) { *p = v; }
-__device__ __forceinline__ float rec_get(const float* p) { return *p; }
+// A lane's records lie in a block of its warp (device scratch, one block per
+// warp of the grid, fields outermost and lanes innermost: a warp's store or
+// load of a field is one 128-byte line); the segment marched again has the
+// block's last kSegRounds rounds.  What a step's level, tap positions and
+// occlusion divisor take is computed again from its distance.
+enum RecField { kRecAlpha, kRecOcc, kRecOp, kRecSlope, kRecColour, kRecCorr, kRecStep, kRecFields };
+constexpr size_t kRecRounds = kStoredRounds + kSegRounds;
+constexpr size_t kRecWarpFloats = (size_t)kRecFields * kRecRounds * 32;
+__device__ __forceinline__ float& rec_at(float* rec, int field, int slot) {
+    return rec[((size_t)field * kRecRounds + slot) * 32 + (threadIdx.x & 31)];
+}
 
 // Diffuse cones per warp group: 0 deals them cone-major (each cone slot over
 // all samples of the coherent order in turn); T > 0 deals all slots of T
@@ -133,130 +146,141 @@ __device__ __forceinline__ float opacity_slope(const StepDetail& e) {
                                                                    : 0.0f;
 }
 
-// One step of trace_cone (same expressions) at march state m: advances m
-// (alpha, occlusion, schedule) and returns the step.
-__device__ __forceinline__ StepDetail march_step(const F4Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
-                                                 const ConeGeo& K,
-                                                 MarchState& m) {
-    const Sched s{m.step, m.seg, m.diameter};
-    const StepDetail e = exact_step_detail(T, C, d, K, s);
-    const float k = clampf(1.0f - m.alpha, 0.0f, 1.0f);
-    m.alpha = m.alpha + k * e.op;
-    m.occ = m.occ + (1.0f - m.occ) * e.op / e.q;
-    Sched n = s;
-    sched_advance(n, K);
-    m.step = n.step;
-    m.seg = n.seg;
-    m.diameter = n.diameter;
-    return e;
+// A group's cone during its walk: one value on all of the group's lanes.
+struct Group {
+    int size, first;  // lanes; the first of them
+    __device__ __forceinline__ int at() const { return (int)(threadIdx.x & 31) - first; }
+};
+
+// One round of trace_cone (same expressions) from march state m, which it
+// advances: each lane samples its step, then the states before the steps
+// follow in step order.  Writes the lane's record to `slot`; false where the
+// cone does not have the lane's step.
+__device__ __forceinline__ bool march_round(const F4Atlas& T, const MarchScale& C, const vct_cone_tracing_desc& d,
+                                            const ConeGeo& K, const Group& g, float3 gC, float max_dist, bool running,
+                                            MarchState& m, float* rec, int slot) {
+    constexpr unsigned kFull = 0xffffffffu;
+    Sched s{m.step, m.seg, m.diameter}, mine = s;
+    for (int j = 0; j < g.size; ++j) {
+        if (g.at() == j) mine = s;
+        sched_advance(s, K);
+    }
+    const bool has = running && mine.step < max_dist;
+    StepDetail e;
+    e.op = e.q = 0.0f;
+    if (has) e = exact_step_detail(T, C, d, K, mine);
+    const uint32_t has_mask = __ballot_sync(kFull, has) >> g.first;
+    float alpha = m.alpha, occ = m.occ, alpha0 = 0.0f, occ0 = 0.0f;
+    bool mine_on = false;
+    for (int j = 0; j < g.size; ++j) {
+        const bool on = ((has_mask >> j) & 1u) && occ < 1.0f;
+        const float op = __shfl_sync(kFull, e.op, g.first + j), q = __shfl_sync(kFull, e.q, g.first + j);
+        if (g.at() == j) {
+            alpha0 = alpha;
+            occ0 = occ;
+            mine_on = on;
+        }
+        if (on) {
+            const float k = clampf(1.0f - alpha, 0.0f, 1.0f);
+            alpha = alpha + k * op;
+            occ = occ + (1.0f - occ) * op / q;
+        }
+    }
+    if (running) m = MarchState{s.step, s.seg, s.diameter, alpha, occ};
+    if (mine_on) {
+        rec_at(rec, kRecAlpha, slot) = alpha0;
+        rec_at(rec, kRecOcc, slot) = occ0;
+        rec_at(rec, kRecOp, slot) = e.op;
+        rec_at(rec, kRecSlope, slot) = opacity_slope(e);
+        rec_at(rec, kRecColour, slot) = (gC.x * e.smp.x + gC.y * e.smp.y + gC.z * e.smp.z) * e.correction;
+        rec_at(rec, kRecCorr, slot) = e.correction;
+        rec_at(rec, kRecStep, slot) = mine.step;
+    }
+    return mine_on;
 }
 
-// The adjoint of one cone per lane: gC (rgb) and gO (d/d occlusion)
-// at the end of the march.  The warp's lanes run in lock step: every loop
-// runs to the warp's longest march and a lane sits out the steps its cone
-// does not have (or all of them when `active` is false).  The reverse walk
-// reads no texels: a stored step's record, or the recompute of a later
-// segment, kept in local arrays.
+// The adjoint of a warp's cones, g.size lanes to each: gC (rgb) and gO (d/d
+// occlusion) at the end of the march.  The warp's lanes run in lock step:
+// every loop runs to the warp's longest march and a lane sits out the steps
+// its cone does not have (or all of them when `active` is false).
 // `rec`: the warp's record block (kRecWarpFloats floats), written and read
-// by each lane for its own cone only.
-__device__ void cone_backward_lane(const F4Atlas& T, float4* __restrict__ G, const MarchScale& C,
-                                   const vct_cone_tracing_desc& d,
-                                   const ConeGeo& K, float3 gC, float gO, bool active, float max_dist,
-                                   float* rec, int* __restrict__ err) {
+// by each lane for its own steps only.
+__device__ void cone_backward(const F4Atlas& T, float4* __restrict__ G, const MarchScale& C,
+                              const vct_cone_tracing_desc& d, const ConeGeo& K, const Group& g, float3 gC, float gO,
+                              bool active, float max_dist, float* rec, int* __restrict__ err) {
     constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     MarchState ckpt[kMaxSegments];
     const Sched s0 = first_sched(K);
     MarchState m{s0.step, s0.seg, s0.diameter, 0.0f, 0.0f};
-    int n = 0;
+    int rounds = 0, mine = 0;  // of the cone, and those in which it has the lane's step (the first ones)
     bool running = active && m.step < max_dist && m.occ < 1.0f;
-    for (int j = 0; __any_sync(kFull, running); ++j) {
-        if ((j % kSegSteps) == 0 && j / kSegSteps >= kMaxSegments) {  // j is warp-uniform
+    for (int j = 0; __any_sync(kFull, running); ++j) {  // j is warp-uniform
+        if (j * g.size >= kMaxSteps) {
             if (running) atomicOr(err, 1);
             return;
         }
-        if (running) {
-            if ((j % kSegSteps) == 0 && j >= kStoredSteps) ckpt[j / kSegSteps] = m;
-            const float alpha0 = m.alpha, occ0 = m.occ, step0 = m.step;
-            const StepDetail e = march_step(T, C, d, K, m);
-            if (j < kStoredSteps) {
-                float* r = rec + (size_t)j * 32 + lane;
-                constexpr size_t F = (size_t)kStoredSteps * 32;  // one field's floats
-                rec_put(r + kRecAlpha * F, alpha0);
-                rec_put(r + kRecOcc * F, occ0);
-                rec_put(r + kRecCorr * F, e.correction);
-                rec_put(r + kRecQ * F, e.q);
-                rec_put(r + kRecOp * F, e.op);
-                rec_put(r + kRecSlope * F, opacity_slope(e));
-                rec_put(r + kRecR * F, e.smp.x);
-                rec_put(r + kRecG * F, e.smp.y);
-                rec_put(r + kRecB * F, e.smp.z);
-                rec_put(r + kRecStep * F, step0);
-                rec_put(r + kRecFr * F, e.fr);
-                rec_put(r + kRecLevels * F, __int_as_float((e.lower & 0xffff) | (e.upper << 16)));
-            }
-            ++n;
-            running = m.step < max_dist && m.occ < 1.0f;
-        }
+        const int past = j - kStoredRounds;
+        if (past >= 0 && past % kSegRounds == 0) ckpt[past / kSegRounds] = m;
+        const int slot = past < 0 ? j : kStoredRounds + past % kSegRounds;
+        mine += march_round(T, C, d, K, g, gC, max_dist, running, m, rec, slot);
+        rounds += running;
+        running = running && m.step < max_dist && m.occ < 1.0f;
     }
-    const int nmax = __reduce_max_sync(kFull, n);
+    const int nmax = __reduce_max_sync(kFull, rounds);
     float gA = 0.0f;
-    MarchState seg[kSegSteps];
-    StepDetail seg_step[kSegSteps];
-    for (int sidx = (nmax - 1) / kSegSteps; nmax > 0 && sidx >= 0; --sidx) {
-        const int first = sidx * kSegSteps, last = min(nmax, first + kSegSteps);
-        const int mine = min(n, first + kSegSteps);  // this lane's steps of the segment: first .. mine - 1
-        if (first < kStoredSteps) {  // warp-uniform: the segment's steps are in the record block
-            for (int i = last - 1; i >= first; --i) {
-                if (i >= mine) continue;
-                const float* rr = rec + (size_t)i * 32 + lane;
-                constexpr size_t F = (size_t)kStoredSteps * 32;
-                const float alpha = rec_get(rr + kRecAlpha * F), occ = rec_get(rr + kRecOcc * F);
-                const float c = rec_get(rr + kRecCorr * F), q = rec_get(rr + kRecQ * F), op = rec_get(rr + kRecOp * F);
-                const float slope = rec_get(rr + kRecSlope * F);
-                const float sr = rec_get(rr + kRecR * F), sg = rec_get(rr + kRecG * F), sb = rec_get(rr + kRecB * F);
-                const float step = rec_get(rr + kRecStep * F), fr = rec_get(rr + kRecFr * F);
-                const int lv = __float_as_int(rec_get(rr + kRecLevels * F));
-                const float k_raw = 1.0f - alpha;
-                const float k = clampf(k_raw, 0.0f, 1.0f);
-                float4 gs;
-                gs.x = gC.x * k * c;
-                gs.y = gC.y * k * c;
-                gs.z = gC.z * k * c;
-                const float gop = gA * k + gO * (1.0f - occ) / q;
-                gs.w = gop * slope;
-                if (k_raw >= 0.0f && k_raw <= 1.0f) gA = gA - ((gC.x * sr + gC.y * sg + gC.z * sb) * c + gA * op);
-                gO = gO * (1.0f - op / q);
-                const float3 pos = K.start + K.dir * step;  // exact_step_detail's expression
-                scatter_step(G, T.A, C, d, K, pos, (int)(short)(lv & 0xffff), lv >> 16, fr, gs);
-            }
-            continue;
+    int kept = (nmax - 1 - kStoredRounds) / kSegRounds;  // the segment whose records the block holds
+    for (int j = nmax - 1; j >= 0; --j) {
+        const int past = j - kStoredRounds, seg = past / kSegRounds;
+        if (past >= 0 && seg != kept) {  // march the segment again
+            MarchState r = ckpt[seg];
+            for (int i = 0; i < kSegRounds; ++i)
+                march_round(T, C, d, K, g, gC, max_dist, kStoredRounds + seg * kSegRounds + i < rounds, r, rec,
+                            kStoredRounds + i);
+            kept = seg;
         }
-        MarchState r;
-        if (first < n) r = ckpt[sidx];
-        for (int i = first; i < last; ++i) {
-            if (i < mine) {
-                seg[i - first] = r;
-                seg_step[i - first] = march_step(T, C, d, K, r);
+        const int slot = past < 0 ? j : kStoredRounds + past % kSegRounds;
+        const bool on = j < mine;
+        float alpha = 0.0f, occ = 0.0f, op = 0.0f, slope = 0.0f, colour = 0.0f, c = 0.0f, q = 1.0f, level = 0.0f;
+        float3 pos = f3(0.f, 0.f, 0.f);
+        if (on) {
+            alpha = rec_at(rec, kRecAlpha, slot);
+            occ = rec_at(rec, kRecOcc, slot);
+            op = rec_at(rec, kRecOp, slot);
+            slope = rec_at(rec, kRecSlope, slot);
+            colour = rec_at(rec, kRecColour, slot);
+            c = rec_at(rec, kRecCorr, slot);
+            const float step = rec_at(rec, kRecStep, slot);
+            // exact_step_detail's expressions
+            pos = K.start + K.dir * step;
+            level = step_level(C, K, pos, j == 0 && g.at() == 0 ? first_sched(K).diameter : step * K.coef);
+            q = 1.0f + (step + K.uvs * exp2f(level)) * d.occlusion_decay;
+        }
+        const float k_raw = 1.0f - alpha, k = clampf(k_raw, 0.0f, 1.0f);
+        const float keep = 1.0f - op / q;
+        const uint32_t on_mask = __ballot_sync(kFull, on) >> g.first;
+        const uint32_t in_mask = __ballot_sync(kFull, k_raw >= 0.0f && k_raw <= 1.0f) >> g.first;
+        float my_gA = 0.0f, my_gO = 0.0f;
+        for (int i = g.size - 1; i >= 0; --i) {
+            const int src = g.first + i;
+            const float op_i = __shfl_sync(kFull, op, src), colour_i = __shfl_sync(kFull, colour, src);
+            const float keep_i = __shfl_sync(kFull, keep, src);
+            if (g.at() == i) {
+                my_gA = gA;
+                my_gO = gO;
+            }
+            if ((on_mask >> i) & 1u) {
+                if ((in_mask >> i) & 1u) gA = gA - (colour_i + gA * op_i);
+                gO = gO * keep_i;
             }
         }
-        for (int i = last - 1; i >= first; --i) {
-            if (i >= mine) continue;
-            const MarchState& mi = seg[i - first];
-            const StepDetail& e = seg_step[i - first];
-            const float c = e.correction;
-            const float k_raw = 1.0f - mi.alpha;
-            const float k = clampf(k_raw, 0.0f, 1.0f);
+        if (on) {
             float4 gs;
             gs.x = gC.x * k * c;
             gs.y = gC.y * k * c;
             gs.z = gC.z * k * c;
-            const float gop = gA * k + gO * (1.0f - mi.occ) / e.q;
-            gs.w = gop * opacity_slope(e);
-            if (k_raw >= 0.0f && k_raw <= 1.0f)
-                gA = gA - ((gC.x * e.smp.x + gC.y * e.smp.y + gC.z * e.smp.z) * c + gA * e.op);
-            gO = gO * (1.0f - e.op / e.q);
-            scatter_step(G, T.A, C, d, K, e.pos, e.lower, e.upper, e.fr, gs);
+            const float gop = my_gA * k + my_gO * (1.0f - occ) / q;
+            gs.w = gop * slope;
+            scatter_step(G, T.A, C, d, K, pos, (int)floorf(level), (int)ceilf(level), fractf(level), gs);
         }
     }
 }
@@ -291,16 +315,21 @@ __global__ void __launch_bounds__(128) k_cone_backward_diffuse(const __grid_cons
                                                                const vct_surface_sample* __restrict__ samples,
                                                                int64_t n, const uint32_t* __restrict__ order,
                                                                const float4* __restrict__ gd, float4* __restrict__ G,
-                                                               float* rec_all, int* __restrict__ err) {
+                                                               float* rec_all, int* __restrict__ err,
+                                                               unsigned int* __restrict__ ticket) {
     const vct_cone_tracing_desc& d = P.d;
     float* rec = rec_all + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRecWarpFloats;
     const bool c32 = d.enable_32_cones != 0;
     const int nc = c32 ? 32 : 16;
     const int lane = threadIdx.x & 31;
     const int64_t total = n * nc;
-    // warp-uniform trip count: a warp's lanes enter cone_backward_lane together
-    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < total;
-         t0 += (int64_t)gridDim.x * blockDim.x) {
+    const Group g1{1, lane};
+    for (;;) {
+        unsigned int item = 0;
+        if (lane == 0) item = atomicAdd(ticket, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        const int64_t t0 = (int64_t)item * 32;
+        if (t0 >= total) break;
         const int64_t t = t0 + lane;
         bool active = t < total;
         // a warp's lanes march the same cone of consecutive samples in the coherent order (the same direction
@@ -332,28 +361,34 @@ __global__ void __launch_bounds__(128) k_cone_backward_diffuse(const __grid_cons
         active = active && diffuse_seeds(P, g, gd[i], cos_t, nc, gC, gO);
         const ConeGeo K = make_cone(d, start, dir, cone_coef(P.diffuse_aperture), min_level,
                                     fmaxf(kMinTraceStepFactor, d.min_trace_step_factor));
-        cone_backward_lane(T, G, C, d, K, gC, gO, active, kMaxTraceDistance, rec, err);
+        cone_backward(T, G, C, d, K, g1, gC, gO, active, kMaxTraceDistance, rec, err);
     }
 }
 
-// One lane per specular cone of the aperture-grouped list (a warp's cones
-// share their step schedule, so the lock-step walk keeps its lanes busy).
+// A group of lanes (cone_group) per specular cone of the aperture-grouped list
+// (a warp's cones share their step schedule, so the lock-step walk keeps its
+// lanes busy).
 __global__ void __launch_bounds__(128) k_cone_backward_specular(
     const __grid_constant__ TraceParams P, const __grid_constant__ MarchScale C, F4Atlas T,
     const vct_surface_sample* __restrict__ samples, const uint32_t* __restrict__ list,
     const unsigned int* __restrict__ spec_count, const float4* __restrict__ gsp, float4* __restrict__ G,
-    float* rec_all, int* __restrict__ err) {
+    float* rec_all, int* __restrict__ err,
+                                                               unsigned int* __restrict__ ticket) {
     const vct_cone_tracing_desc& d = P.d;
     float* rec = rec_all + (size_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRecWarpFloats;
     if (!(d.rendering_mode == 6 || d.rendering_mode >= 8)) return;
     const int lane = threadIdx.x & 31;
     const int64_t m = *spec_count;
-    // warp-uniform trip count: a warp's lanes enter cone_backward_lane together
-    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < m;
-         t0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = t0 + lane;
+    const int group = cone_group(m), cones = 32 / group;
+    const Group gr{group, lane & ~(group - 1)};
+    for (;;) {
+        unsigned int t0 = 0;
+        if (lane == 0) t0 = atomicAdd(ticket, (unsigned)cones);
+        t0 = __shfl_sync(0xffffffffu, t0, 0);
+        if ((int64_t)t0 >= m) break;
+        const int64_t t = (int64_t)t0 + lane / group;
         bool active = t < m;
-        const uint32_t i = __ldg(list + (active ? t : t0));
+        const uint32_t i = __ldg(list + (active ? t : (int64_t)t0));
         const GSample g = load_sample(samples + i, P.eye);
         const float4 GS = gsp[i];
         const float isi = d.indirect_specular_intensity;
@@ -366,7 +401,7 @@ __global__ void __launch_bounds__(128) k_cone_backward_specular(
         const float3 sdir = reflect3(f3(-g.view.x, -g.view.y, -g.view.z), g.normal);
         const ConeGeo K = make_cone(d, start, sdir, cone_coef(fmaxf(g.roughness, kMinSpecularAperture)), min_level,
                                     d.voxel_size);
-        cone_backward_lane(T, G, C, d, K, gC, 0.0f, active, kMaxTraceDistance, rec, err);
+        cone_backward(T, G, C, d, K, gr, gC, 0.0f, active, kMaxTraceDistance, rec, err);
     }
 }
 
@@ -402,7 +437,7 @@ extern "C" int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const 
     VCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k_cone_backward_diffuse, 128, 0));
     VCT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_cone_backward_specular, 128, 0));
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((n * nc + 127) / 128, (int64_t)sms * std::max(occ_d, 1)));
-    const int64_t lblocks = std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, (int64_t)sms * std::max(occ_s, 1)));
+    const int64_t lblocks = std::max<int64_t>(1, std::min<int64_t>((n * kMaxConeGroup + 127) / 128, (int64_t)sms * std::max(occ_s, 1)));
     const size_t rec_bytes = (size_t)std::max(blocks, lblocks) * (128 / 32) * kRecWarpFloats * sizeof(float);
     int* err = nullptr;
     VCT_CUDA_TRY(cudaMallocAsync(&err, sizeof(int), st));
@@ -423,12 +458,13 @@ extern "C" int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const 
     }
     float4* G = reinterpret_cast<float4*>(grad_atlas4);
     k_cone_backward_diffuse<<<(int)blocks, 128, 0, st>>>(P, C, T, samples, n, plan.order,
-                                                          reinterpret_cast<const float4*>(grad_diffuse), G, rec, err);
+                                                          reinterpret_cast<const float4*>(grad_diffuse), G, rec, err,
+                                                          plan.spec_count + 2);
     cudaError_t le = cudaGetLastError();
     if (le == cudaSuccess) {
         k_cone_backward_specular<<<(int)lblocks, 128, 0, st>>>(P, C, T, samples, plan.spec_list, plan.spec_count,
                                                                reinterpret_cast<const float4*>(grad_specular), G, rec,
-                                                               err);
+                                                               err, plan.spec_count + 1);
         le = cudaGetLastError();
     }
     int h_err = 0;
@@ -478,11 +514,11 @@ __global__ void __launch_bounds__(kSqErrThreads) k_sq_error(const float4* __rest
 
 __global__ void k_sq_error_fold(const double* __restrict__ partial, int blocks, double scale,
                                 double* __restrict__ loss) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < blocks; ++b) s += partial[b];
-        *loss = s * scale;
-    }
+    // one warp, lanes over the partial sums in turn, then the lanes in a fixed tree (608 adds in a row took 19 us)
+    double s = 0.0;
+    for (int b = threadIdx.x; b < blocks; b += 32) s += partial[b];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *loss = s * scale;
 }
 
 struct AdamArgs {
