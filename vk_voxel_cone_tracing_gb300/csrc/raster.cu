@@ -713,23 +713,37 @@ struct TilePlan {
 
 // Item of every tile: item i owns tiles [tile_end[i-1], tile_end[i]).  A warp
 // takes 32 items; a lane writes its own item's tiles when there are at most
-// eight, and the warp writes the larger items' together, so an item with
-// thousands of tiles (a floor quad in a 2048^2 shadow map) is spread over the
-// lanes.
-__global__ void k_tile_items(const uint32_t* __restrict__ tile_end, int64_t items, uint32_t* __restrict__ tile_item) {
+// eight, the warp writes the larger items' together, and the block those with
+// thousands (a floor quad has 65,536 in a 2048^2 shadow map: one warp took 68
+// us over it, the kernel's whole time).
+constexpr uint32_t kBlockItemTiles = 1024;
+__global__ void __launch_bounds__(256) k_tile_items(const uint32_t* __restrict__ tile_end, int64_t items,
+                                                    uint32_t* __restrict__ tile_item) {
+    __shared__ uint32_t huge[256];  // block-local numbers of the items the block writes
+    __shared__ uint32_t nhuge;
     const int lane = threadIdx.x & 31;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < items; base += nwarps * 32) {
-        const int64_t i = base + lane;
+    for (int64_t block = (int64_t)blockIdx.x * 256; block < items; block += (int64_t)gridDim.x * 256) {
+        if (threadIdx.x == 0) nhuge = 0u;
+        __syncthreads();
+        const int64_t i = block + threadIdx.x;
         const uint32_t e_i = i < items ? tile_end[i] : 0u;
         const uint32_t b_i = i < items ? (i > 0 ? tile_end[i - 1] : 0u) : 0u;
-        if (e_i - b_i <= 8u)
+        const uint32_t n_i = e_i - b_i;
+        if (n_i <= 8u)
             for (uint32_t g = b_i; g < e_i; ++g) tile_item[g] = (uint32_t)i;
-        for (unsigned big = __ballot_sync(0xffffffffu, e_i - b_i > 8u); big; big &= big - 1u) {
+        if (n_i > kBlockItemTiles) huge[atomicAdd(&nhuge, 1u)] = threadIdx.x;
+        for (unsigned big = __ballot_sync(0xffffffffu, n_i > 8u && n_i <= kBlockItemTiles); big; big &= big - 1u) {
             const int j = __ffs(big) - 1;
             const uint32_t b = __shfl_sync(0xffffffffu, b_i, j), e = __shfl_sync(0xffffffffu, e_i, j);
-            for (uint32_t g = b + (uint32_t)lane; g < e; g += 32u) tile_item[g] = (uint32_t)(base + j);
+            for (uint32_t g = b + (uint32_t)lane; g < e; g += 32u) tile_item[g] = (uint32_t)(i - lane + j);
         }
+        __syncthreads();
+        for (uint32_t k = 0; k < nhuge; ++k) {
+            const int64_t h = block + huge[k];
+            const uint32_t b = h > 0 ? tile_end[h - 1] : 0u, e = tile_end[h];
+            for (uint32_t g = b + threadIdx.x; g < e; g += 256u) tile_item[g] = (uint32_t)h;
+        }
+        __syncthreads();
     }
 }
 
@@ -905,9 +919,8 @@ __device__ inline void sample_bz(const TileSlot& T, int ox, int oy, float b[3], 
     b[2] = (flags & kTileSwapped) ? bo[1] : bo[2];
 }
 
-// Coverage mask of the NS samples of the pixel at offset (ox0, oy0) from the
+// Coverage mask of the 8 samples of the pixel at offset (ox0, oy0) from the
 // tile corner (bit s: sample s covered and inside the depth clip).
-template <int NS>
 __device__ inline uint32_t cover_pixel(const TileTest& t, const TileSlot& T, int ox0, int oy0) {
     uint32_t mask = 0;
     if (t.flags & kTileSmall) {
@@ -915,18 +928,18 @@ __device__ inline uint32_t cover_pixel(const TileTest& t, const TileSlot& T, int
 #pragma unroll
         for (int i = 0; i < 3; ++i) base[i] = t.e[i] + (t.dx[i] * oy0 - t.dy[i] * ox0);
 #pragma unroll
-        for (int s = NS - 1; s >= 0; --s) {
-            const int ox = NS == 1 ? 128 : sample_x(s), oy = NS == 1 ? 128 : sample_y(s);
+        for (int s = 7; s >= 0; --s) {
+            const int ox = sample_x(s), oy = sample_y(s);
             int x = 0;
 #pragma unroll
             for (int i = 0; i < 3; ++i) x |= base[i] + (t.dx[i] * oy - t.dy[i] * ox);
             mask = __funnelshift_l((uint32_t)x, mask, 1);  // the sign bit in: 1 = outside
         }
-        mask = ~mask & ((1u << NS) - 1u);
+        mask = ~mask & 0xffu;
     } else {
 #pragma unroll 1
-        for (int s = 0; s < NS; ++s) {
-            const int ox = ox0 + (NS == 1 ? 128 : c_sample_loc8[s][0]), oy = oy0 + (NS == 1 ? 128 : c_sample_loc8[s][1]);
+        for (int s = 0; s < 8; ++s) {
+            const int ox = ox0 + c_sample_loc8[s][0], oy = oy0 + c_sample_loc8[s][1];
             bool cov = true;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -940,10 +953,57 @@ __device__ inline uint32_t cover_pixel(const TileTest& t, const TileSlot& T, int
         for (uint32_t m = mask; m; m &= m - 1u) {
             const int s = __ffs(m) - 1;
             float b[3], z;
-            sample_bz(T, ox0 + (NS == 1 ? 128 : c_sample_loc8[s][0]), oy0 + (NS == 1 ? 128 : c_sample_loc8[s][1]), b, z);
+            sample_bz(T, ox0 + c_sample_loc8[s][0], oy0 + c_sample_loc8[s][1], b, z);
             if (!(z >= 0.0f && z <= 1.0f)) mask &= ~(1u << s);
         }
     return mask;
+}
+
+// The centre samples of `count` pixels of a tile from its pixel `lp` on, for
+// the one-sample passes: the edge values step from pixel to pixel (V: 32 bits
+// where the tile's values fit them), the covered test and the depth are
+// cover_pixel's and sample_bz's.
+template <int KIND, class V>
+__device__ __forceinline__ void centre_run(const RasterArgs& A, const TileSlot& T, uint32_t lp, uint32_t count) {
+    const uint32_t tw = (uint32_t)T.tw, flags = T.test.flags;
+    const uint32_t row = tw > 1u ? __umulhi(lp, T.tw_magic) : lp;
+    uint32_t col = lp - row * tw;
+    const int ox = (int)col * 256 + 128, oy = (int)row * 256 + 128;
+    V e[3], right[3], down[3];
+    float zi[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const V dx = (V)T.dX[i], dy = (V)T.dY[i];
+        e[i] = (V)T.E[i] + (dx * oy - dy * ox);
+        right[i] = -dy * 256;
+        down[i] = dx * 256 + dy * (256 * (int)(tw - 1u));  // from a row's last pixel to the next row's first
+        zi[i] = T.z[i];
+    }
+    const float inv_area = T.inv_area;
+    int64_t at = (int64_t)(T.ty + (int)row) * A.W + (T.tx + (int)col);
+    for (;;) {
+        V out = 0;  // negative: outside an edge
+#pragma unroll
+        for (int i = 0; i < 3; ++i) out |= e[i] - (V)(((flags >> i) & 1u) ^ 1u);
+        if (out >= 0) {
+            const float z = ((float)e[0] * inv_area * zi[0] + (float)e[1] * inv_area * zi[1]) +
+                            (float)e[2] * inv_area * zi[2];
+            if ((flags & kTileZsafe) || (z >= 0.0f && z <= 1.0f)) {
+                if (KIND == K_SHADOW) {
+                    atomicMin(reinterpret_cast<unsigned int*>(A.depth) + at, __float_as_uint(z));
+                } else if (z < 1.0f) {  // depth test LESS against the cleared 1.0
+                    // z >= 0 here; -0 is keyed as +0 so the bit order is the numeric order
+                    atomicMin(A.vis + at, ((unsigned long long)(__float_as_uint(z) & 0x7fffffffu) << 32) | T.item);
+                }
+            }
+        }
+        if (--count == 0u) break;
+        const bool next_row = ++col == tw;
+        if (next_row) col = 0u;
+        at += next_row ? A.W - (int)tw + 1 : 1;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) e[i] += next_row ? down[i] : right[i];
+    }
 }
 
 // The covered samples of a warp's 32 pixels (lane i's pixel has coverage
@@ -1017,7 +1077,8 @@ static int chunk_group(bool one_sample, uint32_t tiles) {
 // edges, which bounds the kernel on small triangles.  With the sign-bit tests,
 // 32-bit edge values, the reduction instead of a binary search per pixel and
 // the slots' stride: 1M-triangle hall at R = 256, opacity + count 1.76 -> 0.95
-// ms, emission 0.85 -> 0.51, shadow 0.81 -> 0.59; octree count and emission of
+// ms, emission 0.85 -> 0.51, shadow 0.81 -> 0.59 (and, with its edge values
+// stepped from pixel to pixel in centre_run, 0.50); octree count and emission of
 // the 4M-triangle terrain 1.12 -> 0.53 and 1.48 -> 1.01 ms.
 //   P_DIRECT writes the pass's output (opacity, shadow depth, atomic injection);
 //   P_COUNT counts covered samples and their records per tile;
@@ -1030,7 +1091,6 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                                                uint32_t* __restrict__ counts,
                                                const unsigned long long* __restrict__ offs, FragDesc* __restrict__ frags,
                                                int* __restrict__ err) {
-    constexpr int NS = (KIND == K_SHADOW || KIND == K_GBUFFER) ? 1 : 8;
     constexpr bool RANKED = PHASE != P_DIRECT;
     // the opacity writes run over the round's covered samples dealt to the lanes
     constexpr bool FLAT_OPACITY = (KIND == K_OPACITY || KIND == K_OPA_COUNT) && PHASE != P_WRITE;
@@ -1107,8 +1167,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
         int cj = -1;
         if (KIND == K_SHADOW || KIND == K_GBUFFER) {
             // one centre sample per pixel: each lane takes four consecutive
-            // pixels of the list per round, so the tile search and slot reload
-            // are shared by four depth tests
+            // pixels of the list per round, in runs of one tile
             for (uint32_t q0 = (uint32_t)lane * 4u; q0 < P; q0 += 128u) {
                 int lo = 0, hi = 31;
                 while (lo < hi) {
@@ -1116,29 +1175,14 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                     if (S[mid].px_end > q0) hi = mid;
                     else lo = mid + 1;
                 }
-                int j = lo;
-                for (uint32_t q = q0; q < q0 + 4u && q < P; ++q) {
-                    while (S[j].px_end <= q) ++j;  // the next pixel's tile (at most 3 steps)
-                    if (j != cj) {
-                        t = S[j].test;
-                        cj = j;
-                    }
-                    const uint32_t lp = q - S[j].px_start, tw = (uint32_t)S[j].tw;
-                    const uint32_t row = tw > 1u ? __umulhi(lp, S[j].tw_magic) : lp;
-                    const int ox0 = (int)(lp - row * tw) * 256, oy0 = (int)row * 256;
-                    if (cover_pixel<1>(t, S[j], ox0, oy0)) {
-                        float b[3], z;
-                        sample_bz(S[j], ox0 + 128, oy0 + 128, b, z);
-                        const int px = S[j].tx + (ox0 >> 8), py = S[j].ty + (oy0 >> 8);
-                        if (KIND == K_SHADOW) {
-                            atomicMin(reinterpret_cast<unsigned int*>(A.depth) + (int64_t)py * A.W + px,
-                                      __float_as_uint(z));
-                        } else if (z < 1.0f) {  // depth test LESS against the cleared 1.0
-                            // z >= 0 here; -0 is keyed as +0 so the bit order is the numeric order
-                            atomicMin(A.vis + (int64_t)py * A.W + px,
-                                      ((unsigned long long)(__float_as_uint(z) & 0x7fffffffu) << 32) | S[j].item);
-                        }
-                    }
+                const uint32_t qe = min(q0 + 4u, P);
+                for (uint32_t q = q0; q < qe; ++lo) {
+                    const TileSlot& T = S[lo];
+                    const uint32_t e = min(qe, T.px_end);
+                    if (e <= q) continue;  // a tile without pixels
+                    if (T.test.flags & kTileNear) centre_run<KIND, int>(A, T, q - T.px_start, e - q);
+                    else centre_run<KIND, long long>(A, T, q - T.px_start, e - q);
+                    q = e;
                 }
             }
             __syncwarp();
@@ -1166,7 +1210,7 @@ __global__ void __launch_bounds__(128, 6) k_cover(const __grid_constant__ Raster
                 const uint32_t row = tw > 1u ? __umulhi(lp, S[j].tw_magic) : lp;
                 ox0 = (int)(lp - row * tw) * 256;
                 oy0 = (int)row * 256;
-                mask = cover_pixel<NS>(t, S[j], ox0, oy0);
+                mask = cover_pixel(t, S[j], ox0, oy0);
                 if (KIND == K_INJECT && PHASE == P_DIRECT) {
                     const TileSlot& T = S[j];
                     const int lvl = (int)(T.meta & 7u);
