@@ -77,3 +77,34 @@ def test_edges_around_the_32_bit_limits(cuda, oracle):
     passes.voxelize_opacity(ds, regions, R, atlas, ws, level_mask=0x5)
     want = oracle.voxelize_opacity(scene, R, clipmap.regions_to_numpy(regions), level_mask=0x5)
     assert np.array_equal(atlas.cpu().numpy().view(np.uint32), want)
+
+
+def test_triangles_about_the_depth_limits(cuda, oracle):
+    """Triangles facing each axis at depths on both sides of each clip level's near and far limits, from an ulp to
+    a voxel away, flat and tilted across: the ones culled as a whole leave the atlases the oracle's."""
+    torch = cuda
+    from vk_voxel_cone_tracing_gb300 import clipmap, passes
+    from vk_voxel_cone_tracing_gb300.scene import _pack
+    rng = np.random.default_rng(8)
+    R = 32
+    regions = clipmap.clip_regions((0.3, 1.2, -0.6), R)
+    reg = clipmap.regions_to_numpy(regions)
+    tris = []
+    for level in (0, 2):
+        vs = float(reg[level, 6:7].view(np.float32)[0])
+        lo = reg[level, 0:3].astype(np.float64) * vs
+        size = R * vs
+        for axis in range(3):
+            for limit in (lo[axis], lo[axis] + size, lo[axis] + 0.1, lo[axis] + size - 0.1, lo[axis] - 0.1):
+                for off in (0.0, 1e-7, -1e-7, 1e-5, -1e-5, 1e-3, -1e-3, vs, -vs):
+                    c = lo + size * rng.uniform(0.2, 0.8, 3)
+                    c[axis] = limit + off
+                    e = rng.normal(size=(2, 3)) * size * 0.1
+                    e[:, axis] = 0.0 if rng.random() < 0.6 else rng.normal(size=2) * 1e-5
+                    tris.append([c, c + e[0], c + e[1]])
+    scene = _pack(np.array(tris, np.float32), rng)
+    ds, ws = passes.DeviceScene(scene), passes.Workspace()
+    opacity = clipmap.new_atlas(R)
+    passes.voxelize_opacity(ds, regions, R, opacity, ws)
+    want = oracle.voxelize_opacity(scene, R, reg)
+    assert np.array_equal(opacity.cpu().numpy().view(np.uint32), want) and want.any()

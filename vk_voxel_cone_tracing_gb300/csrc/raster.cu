@@ -259,6 +259,20 @@ struct RSetup {
 
 __device__ inline long long floor_div256(long long v) { return v >= 0 ? v / 256 : -((-v + 255) / 256); }
 
+// All three depths so far on one side of the clip that every covered sample's
+// depth is outside it: the samples' weights are >= 0 and sum to 1 within
+// (1 + 2^-24)^3, their depth takes five more roundings (see TileTest), so
+// three depths above 1 + 2^-20 give a depth above 1, and three below zero
+// (by more than what a product with a weight of a third can lose) one below 0.
+// Such a triangle has no tiles.  Most of a scene's triangles are culled so in
+// a fine clip level, whose depth range they miss while its square they meet:
+// opacity + count of the 1M-triangle hall at R = 256 0.95 -> 0.64 ms, emission
+// 0.50 -> 0.46.
+__device__ inline bool depth_culled(float z0, float z1, float z2) {
+    const float hi = 1.00000095367431640625f, lo = -1e-30f;
+    return (z0 > hi && z1 > hi && z2 > hi) || (z0 < lo && z1 < lo && z2 < lo);
+}
+
 __device__ inline RSetup raster_setup(const float4 c[3], int W, int H) {
     RSetup r;
     const float hw = (float)W * 0.5f, hh = (float)H * 0.5f;
@@ -269,7 +283,7 @@ __device__ inline RSetup raster_setup(const float4 c[3], int W, int H) {
         Y[k] = __float2ll_rn((hh * c[k].y + hh) * 256.0f);
     }
     long long area = (X[1] - X[0]) * (Y[2] - Y[0]) - (Y[1] - Y[0]) * (X[2] - X[0]);
-    r.ok = area != 0;
+    r.ok = area != 0 && !depth_culled(c[0].z, c[1].z, c[2].z);
     if (!r.ok) return r;
     // counter-clockwise vertex order: swap vertices 1 and 2 of a clockwise triangle
     const bool sw = area < 0;
@@ -949,13 +963,38 @@ __device__ inline uint32_t cover_pixel(const TileTest& t, const TileSlot& T, int
             mask |= (uint32_t)cov << s;
         }
     }
-    if (!(t.flags & kTileZsafe))
+    if ((t.flags & (kTileZsafe | kTileNear)) == kTileNear) {
+        // the depths of all eight samples in a row: testing the covered ones
+        // one after the other, each with its loads, cost the octree passes
+        // (whose depths are all 1) 0.53 instead of 0.44 and 1.00 instead of 0.89
+        // ms on the 4M-triangle terrain
+        int base[3], dx[3], dy[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            dx[i] = (int)T.dX[i];
+            dy[i] = (int)T.dY[i];
+            base[i] = (int)T.E[i] + (dx[i] * oy0 - dy[i] * ox0);
+        }
+        const float z0 = T.z[0], z1 = T.z[1], z2 = T.z[2], inv_area = T.inv_area;
+        uint32_t in = 0;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const int ox = sample_x(s), oy = sample_y(s);
+            float b[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) b[i] = (float)(base[i] + (dx[i] * oy - dy[i] * ox)) * inv_area;
+            const float z = (b[0] * z0 + b[1] * z1) + b[2] * z2;
+            in |= (uint32_t)(z >= 0.0f && z <= 1.0f) << s;
+        }
+        mask &= in;
+    } else if (!(t.flags & kTileZsafe)) {
         for (uint32_t m = mask; m; m &= m - 1u) {
             const int s = __ffs(m) - 1;
             float b[3], z;
             sample_bz(T, ox0 + c_sample_loc8[s][0], oy0 + c_sample_loc8[s][1], b, z);
             if (!(z >= 0.0f && z <= 1.0f)) mask &= ~(1u << s);
         }
+    }
     return mask;
 }
 
