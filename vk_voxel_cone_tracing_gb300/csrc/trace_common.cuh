@@ -45,8 +45,18 @@ struct TraceParams {
     vct_directional_light_shadow_desc shadow_desc;
     const float* shadow;  // may be null: visibility 1
     int shadow_w, shadow_h;
+    float shadow_wf, shadow_hf, shadow_sx, shadow_sy;  // the sizes and 1 / size as floats (set_shadow_size)
     float diffuse_aperture;  // the diffuse cones' aperture: the shader's constant unless an option sets it
 };
+
+inline void set_shadow_size(TraceParams& p, int w, int h) {
+    p.shadow_w = w;
+    p.shadow_h = h;
+    p.shadow_wf = (float)w;
+    p.shadow_hf = (float)h;
+    p.shadow_sx = w > 0 ? 1.0f / (float)w : 0.0f;
+    p.shadow_sy = h > 0 ? 1.0f / (float)h : 0.0f;
+}
 
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
@@ -90,6 +100,25 @@ __device__ __forceinline__ float shadow_tap(const float* __restrict__ depth, int
     return r0 + (r1 - r0) * b;
 }
 
+// The sum of the sixteen taps of a 5 x 5 texel window, row by row.
+template <class Texel>
+__device__ __forceinline__ float window_sum(const float a[4], const float b[4], const Texel& texel) {
+    float prev[4], sum = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+        float t[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) t[c] = texel(r, c);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float cur = t[c] + (t[c + 1] - t[c]) * a[c];
+            if (r > 0) sum += prev[c] + (cur - prev[c]) * b[r - 1];
+            prev[c] = cur;
+        }
+    }
+    return sum;
+}
+
 // calcVisibility + calcShadowCoefficientPCF16 (shadow.glsl:8-36).
 //
 // The sixteen taps lie one texel apart, so where their four columns and four
@@ -102,6 +131,11 @@ __device__ __forceinline__ float shadow_tap(const float* __restrict__ depth, int
 // were bound by these loads: the octree chain of a 4M-triangle terrain (58.4 M
 // shaded fragments) went from 15.75 to 14.54 ms, the R = 256 frame of the
 // 1M-triangle hall (12.8 M) from 9.55 to 9.28 ms.
+// INSIDE: a copy of the window's code without bounds tests for windows inside
+// the map, which the shading passes gain by (octree shading of the terrain's
+// 57 M samples 1.00 -> 0.93 ms) and the traces' kernels, larger already, lose
+// by (diffuse cones of 131,071 samples 221 -> 230 us).
+template <bool INSIDE = false>
 __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp) {
     if (!p.shadow) return 1.0f;
     const float* V = p.shadow_desc.view;
@@ -111,7 +145,7 @@ __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp
     float px = P[0] * lx + P[4] * ly + P[8] * 0.0f + P[12] * 1.0f;
     float py = P[1] * lx + P[5] * ly + P[9] * 0.0f + P[13] * 1.0f;
     float sx = px * 0.5f + 0.5f, sy = py * 0.5f + 0.5f;
-    float scx = 1.0f / (float)p.shadow_w, scy = 1.0f / (float)p.shadow_h;
+    const float scx = p.shadow_sx, scy = p.shadow_sy;
     const int W = p.shadow_w, H = p.shadow_h;
     int i0 = 0, j0 = 0;
     bool window = true;
@@ -119,7 +153,7 @@ __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const float o = -1.5f + (float)k;
-        const float u = (sx + o * scx * 1.0f) * (float)W - 0.5f, v = (sy + o * scy * 1.0f) * (float)H - 0.5f;
+        const float u = (sx + o * scx * 1.0f) * p.shadow_wf - 0.5f, v = (sy + o * scy * 1.0f) * p.shadow_hf - 0.5f;
         const float fu = floorf(u), fv = floorf(v);
         a[k] = u - fu;
         b[k] = v - fv;
@@ -131,22 +165,13 @@ __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp
     float sum = 0.0f;
     if (window) {
         if (i0 + 4 < 0 || j0 + 4 < 0 || i0 >= W || j0 >= H) return 0.0f;
-        float prev[4];
-#pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            const int j = j0 + r;
-            const float* row = p.shadow + (int64_t)j * W + i0;
-            float t[5];
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                t[c] = (unsigned)j < (unsigned)H && (unsigned)(i0 + c) < (unsigned)W ? __ldg(row + c) : 0.0f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float cur = t[c] + (t[c + 1] - t[c]) * a[c];
-                if (r > 0) sum += prev[c] + (cur - prev[c]) * b[r - 1];
-                prev[c] = cur;
-            }
-        }
+        if (INSIDE && i0 >= 0 && j0 >= 0 && i0 + 4 < W && j0 + 4 < H)
+            sum = window_sum(a, b, [&](int r, int c) { return __ldg(p.shadow + (int64_t)(j0 + r) * W + i0 + c); });
+        else
+            sum = window_sum(a, b, [&](int r, int c) {
+                const bool in = (unsigned)(j0 + r) < (unsigned)H && (unsigned)(i0 + c) < (unsigned)W;
+                return in ? __ldg(p.shadow + (int64_t)(j0 + r) * W + i0 + c) : 0.0f;
+            });
         return sum * 0.0625f;
     }
     for (int yi = 0; yi < 4; ++yi)

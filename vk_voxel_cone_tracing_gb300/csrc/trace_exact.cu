@@ -271,12 +271,11 @@ int fill_trace_params(TraceParams& P, const vct_cone_tracing_desc* desc, const v
         VCT_CHECK_ARG(shadow->width > 0 && shadow->height > 0 && shadow->width <= 32768 && shadow->height <= 32768,
                       "cone trace: bad shadow map size");
         P.shadow = shadow->depth;
-        P.shadow_w = shadow->width;
-        P.shadow_h = shadow->height;
+        set_shadow_size(P, shadow->width, shadow->height);
         P.shadow_desc = *light_shadow;
     } else {
         P.shadow = nullptr;
-        P.shadow_w = P.shadow_h = 0;
+        set_shadow_size(P, 0, 0);
         memset(&P.shadow_desc, 0, sizeof(P.shadow_desc));
     }
     return VCT_OK;
