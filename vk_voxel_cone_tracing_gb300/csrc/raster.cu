@@ -1041,6 +1041,23 @@ __device__ __forceinline__ void centre_run(const RasterArgs& A, const TileSlot& 
     }
 }
 
+// Position of the r-th (from 0) set bit of a mask with more than r set bits
+// among its lowest eight: halves of the mask by their counts
+// (__fns on the 32-bit mask: emission of the 4M-triangle terrain 0.89 instead
+// of 0.84 ms, opacity + count of the 1M-triangle hall 0.64 instead of 0.62).
+__device__ __forceinline__ int nth_bit8(uint32_t m, uint32_t r) {
+    int at = 0;
+#pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+        const uint32_t low = (uint32_t)__popc(m & ((1u << half) - 1u));
+        const bool up = r >= low;
+        r -= up ? low : 0u;
+        m >>= up ? half : 0;
+        at += up ? half : 0;
+    }
+    return at;
+}
+
 // The covered samples of a warp's 32 pixels (lane i's pixel has coverage
 // mask `mask`), dealt one per lane in (pixel, sample) order, 32 per round:
 // fn(valid, o, s, r) runs on every lane (valid false on the lanes past the
@@ -1067,7 +1084,7 @@ __device__ __forceinline__ void for_each_covered(uint32_t mask, int lane, Fn&& f
         o = min(o, 31);
         const uint32_t mo = __shfl_sync(FULL, mask, o), r = k - __shfl_sync(FULL, excl, o);
         const bool valid = k < total;
-        fn(valid, o, valid ? (int)__fns(mo, 0u, (int)r + 1) : 0, r);
+        fn(valid, o, valid ? nth_bit8(mo, r) : 0, r);
     }
 }
 
