@@ -511,9 +511,9 @@ def run_ours(args, world, rank, local):
             cpu = {"value": rate, "unit": "cone samples/s", "cores": cores, "kind": "port",
                    "sample": f"first {ncpu} of {n} samples ({st} cone samples, {dt:.1f} s) traced by the FP32 C++ "
                              "restatement on the same clipmap"}
-        # kernels launched per trace step: Morton keys, cub radix sort of 30 bits (histogram, exclusive sum,
-        # 4 onesweep passes), specular list, diffuse, specular (the texture refresh is a memcpy, not a kernel)
-        launches = 1 if tex is None else 10
+        # kernels launched per trace step: Morton keys, cub radix sort of 24 bits (histogram, exclusive sum,
+        # 3 onesweep passes), specular list, diffuse, specular (the texture refresh is a memcpy, not a kernel)
+        launches = 1 if tex is None else 9
         line = {
             "metric": METRIC, "value": value, "unit": "cone samples/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
@@ -524,7 +524,7 @@ def run_ours(args, world, rank, local):
                        "form": args.form, "R": R, "samples_per_step": n, "cone_samples_per_step": cone_samples,
                        "l2": "inputs larger than L2 (2.47 GB clipmap)",
                        "texture_full_copy_ms": refresh_ms, "trace_tuning": tuning,
-                       "texture": "kept current by the frame's copy-alpha and mip passes" if frame_tex is not None
+                       "texture": "kept current by the frame's radiance fill and mip passes" if frame_tex is not None
                        else ("kept current by the frame's FP16 conversion and FP16 mip passes" if tex is not None
                              else "none (linear atlas)"),
                        "voxelize_inject_mip_ms": frame_ms, "frame_r8_opacity": opacity_r8,
@@ -895,9 +895,8 @@ def large_svo(dev, reps: int, level: int = 9, n_samples: int = 4 << 20, seed: in
     torch.cuda.synchronize()
     cone_samples = int(steps.item())
     trace_ms = statistics.median(events_ms(stream, trace, reps)[0])
-    # algorithmic bytes of the build: the fragment (8 B) + every node on its root-to-leaf path (8 B per
-    # level, summed over the L flag passes: 8 L (L + 1) / 2) + the leaf read-modify-write (8 B)
-    build_bytes = F * (8 + 8 * level * (level + 1) // 2 + 8)
+    # algorithmic bytes of the build: every fragment read once and every node written once, 8 B each
+    build_bytes = 8 * (F + int(nodes.value))
     return {"scene": f"terrain ({sc.triangle_count} fp32 triangles: gradient-noise heightfield + 10000 boxes)",
             "level": level, "resolution": 1 << level, "fragments": F, "nodes": int(nodes.value),
             "pool_capacity_nodes": pool_cap, "fragments_ms": frag_ms, "build_ms": build_ms,
@@ -905,7 +904,7 @@ def large_svo(dev, reps: int, level: int = 9, n_samples: int = 4 << 20, seed: in
             "build_algorithmic_gbs": build_bytes / (build_ms * 1e-3) / 1e9,
             "trace": {"samples": n_samples, "cone_samples": cone_samples, "ms": trace_ms,
                       "cone_samples_per_s": cone_samples / (trace_ms * 1e-3)},
-            "note": "deterministic build (scan allocation, fragment-order leaf fold); CUDA events, median"}
+            "note": "deterministic build (one sort of fragment runs by path, fragment-order leaf fold); CUDA events, median"}
 
 
 def differentiable_volume(dev, R: int = 128, views: int = 16, res: int = 512, seed: int = 5, fit_iterations: int = 8):
@@ -988,8 +987,8 @@ def differentiable_volume(dev, R: int = 128, views: int = 16, res: int = 512, se
             "mips_ms": mips_ms, "mips_backward_ms": mips_bwd_ms,
             "fit": fit_result,
             "note": "float RGBA atlas (16 B per texel, 1.27 GB at R = 128), software trilinear; the adjoint "
-                    "marches each cone once, keeping its first 128 steps' records in device scratch (later segments "
-                    "recomputed from 32-step checkpoints), and scatters float4 atomics"}
+                    "marches each cone once, keeping 48 rounds of steps' records in device scratch (later segments "
+                    "recomputed from 32-round checkpoints), and scatters float4 atomics"}
 
 
 def profile_case(args):

@@ -18,7 +18,7 @@
  * non-blocking stream and two events for that thread, kept until the thread
  * ends: the specular cones run on it beside the diffuse kernel, joined back
  * to the caller's stream before the call returns.  A raster workspace
- * (vct_workspace) likewise creates a side stream, two events and a second
+ * (vct_workspace) likewise creates two side streams, four events and a second
  * workspace on first use by vct_clipmap_frame.
  * vct_cone_trace_fast_noalloc never calls cudaMalloc: its scratch is a static
  * device array that the runtime commits when the array's module loads (see
@@ -294,10 +294,11 @@ int vct_wrap_border(uint32_t* atlas, const vct_border_wrapping_desc* desc, void*
  * sample) like the pass's two attachments.  `cone_steps` (optional, may be
  * NULL) receives += the number of traceCone loop iterations executed.
  * Exact form: FP32 arithmetic, trilinear weights in FP32 (no 8-bit filter
- * weights), reads the linear atlas.  One thread per sample; the samples are
- * walked in a coherent order (normal class, then Morton code of the
- * position; stream-ordered scratch of 24 B per sample), which changes no
- * output. */
+ * weights), reads the linear atlas.  The samples are walked in a coherent
+ * order (normal class, then Morton code of the position), their diffuse cones
+ * dealt to the lanes of a warp, their specular cones listed by aperture and
+ * marched by one to eight lanes each (stream-ordered scratch of 32 B per
+ * sample and the sorts' own), which changes no output. */
 int vct_cone_trace(const vct_cone_tracing_desc* desc, const vct_cam_matrix* cam,
                    const uint32_t* radiance_atlas, int32_t clipmap_resolution,
                    const vct_shadow_map* shadow, const vct_directional_light_desc* light,
@@ -324,8 +325,8 @@ int vct_cone_trace_f32(const vct_cone_tracing_desc* desc, const vct_cam_matrix* 
  * each).  The number of march steps (the occlusion stop) and the clamps are
  * held at their forward values.  Synchronises `stream`; VCT_E_OVERFLOW if a
  * cone marches more than 8192 steps.  Its stream-ordered scratch includes the
- * march records of the first 128 steps of each resident warp's cones
- * (192 KiB per warp: about 480 MB on a 152-SM GPU). */
+ * march records of 80 rounds of steps of each resident warp's cones
+ * (70 KiB per warp: about 174 MB on a 152-SM GPU). */
 int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const vct_cam_matrix* cam, const float* atlas4,
                             int32_t R, const vct_shadow_map* shadow, const vct_directional_light_desc* light,
                             const vct_directional_light_shadow_desc* light_shadow,

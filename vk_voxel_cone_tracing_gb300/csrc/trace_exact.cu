@@ -13,7 +13,7 @@
 // the shader traces it (every rendering mode), the diffuse cones likewise.
 //
 // What bounds it: instructions (57 a texel before the packed lerps, the
-// two-instruction decode and the known divisors of trace_exact.cuh, 25 now;
+// three-instruction decode and the known divisors of trace_exact.cuh, 35 now;
 // half the issue slots are still lost to fetching the loop's code) and, for
 // the specular cones, the length of the longest march: 65,536 cones on one
 // lane each are 13 warps an SM, nearly all of them done when the longest are
