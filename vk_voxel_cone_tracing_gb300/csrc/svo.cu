@@ -235,6 +235,37 @@ __device__ __forceinline__ uint32_t avg_fold_int(uint32_t cur, uint32_t v) {
     return (((uint32_t)cw & 0xffu) << 24) | ((z & 0xffu) << 16) | ((y & 0xffu) << 8) | (x & 0xffu);
 }
 
+// The same steps on a cell whose bytes stay floats: a byte of the fragment is
+// the low bits of 2^23 + byte, a floor is a sum rounded down at 2^23, so no
+// step converts.  A step to or from alpha 0 (the first, the one after the
+// 256-count wraps, a fragment of alpha 0, whose quotient may pass 255) goes by
+// the words.  The conversions bound the emission of the terrain's 57 M
+// fragments: 656 -> 534 us.
+struct LeafCell {
+    float r, g, b, a;
+};
+__device__ __forceinline__ float byte_float(uint32_t v, int k) {
+    return __uint_as_float(__byte_perm(v, 0x4b000000u, 0x7440 + k)) - 8388608.0f;
+}
+__device__ __forceinline__ LeafCell leaf_cell(uint32_t v) {
+    return LeafCell{byte_float(v, 0), byte_float(v, 1), byte_float(v, 2), byte_float(v, 3)};
+}
+__device__ __forceinline__ uint32_t leaf_word(const LeafCell& c) {
+    return ((uint32_t)c.a << 24) | ((uint32_t)c.b << 16) | ((uint32_t)c.g << 8) | (uint32_t)c.r;
+}
+__device__ __forceinline__ void leaf_step(LeafCell& c, uint32_t v) {
+    if (c.a == 0.0f || (v >> 24) == 0u) {
+        c = leaf_cell(avg_fold_int(leaf_word(c), v));
+        return;
+    }
+    const LeafCell f = leaf_cell(v);
+    const float cw = c.a + f.a, inv = __fdividef(1.0f, cw);
+    c.r = __fadd_rd((c.r * c.a + (f.r + 0.5f)) * inv, 8388608.0f) - 8388608.0f;
+    c.g = __fadd_rd((c.g * c.a + (f.g + 0.5f)) * inv, 8388608.0f) - 8388608.0f;
+    c.b = __fadd_rd((c.b * c.a + (f.b + 0.5f)) * inv, 8388608.0f) - 8388608.0f;
+    c.a = cw >= 256.0f ? cw - 256.0f : cw;
+}
+
 // A fragment the light test discarded adds (0, 0, 0, 0): that leaves a cell
 // with alpha as it is and empties one without (0 / 0 stores 0).
 __device__ __forceinline__ uint32_t avg_fold_zero(uint32_t cur) { return (cur >> 24) ? cur : 0u; }
@@ -322,6 +353,7 @@ __global__ void __launch_bounds__(kTreeBlock) k_tree_emit(uint2* __restrict__ po
         }
         uint32_t cell = 0u;
         if (fragments < kLongLeaf) {
+            LeafCell lc{0.0f, 0.0f, 0.0f, 0.0f};
             for (uint32_t h = h0; h < h1; ++h) {
                 const uint32_t run = order[h], e = starts[run + 1];
                 // the fold is a serial chain; fetch four fragments ahead of it
@@ -331,9 +363,10 @@ __global__ void __launch_bounds__(kTreeBlock) k_tree_emit(uint2* __restrict__ po
                     for (int u = 0; u < 4; ++u) v[u] = i + u < e ? __ldg(&frags[i + u].y) & 0xfffffffu : 0u;
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (i + u < e) cell = avg_fold_int(cell, v[u]);
+                        if (i + u < e) leaf_step(lc, v[u]);
                 }
             }
+            cell = leaf_word(lc);
         }
         for (unsigned b = __ballot_sync(0xffffffffu, fragments >= kLongLeaf); b; b &= b - 1u) {
             const int o = __ffs(b) - 1;
