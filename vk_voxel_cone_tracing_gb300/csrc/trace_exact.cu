@@ -311,9 +311,8 @@ int exact_plan(const vct_surface_sample* samples, int64_t n, const vct_cone_trac
     plan->block = b;
     plan->order_block = so.block;
     plan->order = so.order;
-    if (!plan->order) {
-        const uint32_t zero = 0;
-        e = cudaMemcpyAsync(identity, &zero, sizeof(zero), cudaMemcpyHostToDevice, st);
+    if (!plan->order) {  // (a fill, not a copy from the host: a captured copy would read this frame's stack at replay)
+        e = cudaMemsetAsync(identity, 0, sizeof(uint32_t), st);
         plan->order = identity;
     }
     // the specular count and the tickets of the specular and diffuse kernels
