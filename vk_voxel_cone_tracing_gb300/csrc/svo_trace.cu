@@ -22,8 +22,9 @@
 //     division and logarithm only within 2^-16 of a power of two;
 //   * the diffuse cones' level by step comes from a table (the schedule is the
 //     same for all of them);
-//   * a step whose two nodes are zero leaves the composite as it is, so level
-//     size, opacity power and divisions run for the others alone.
+//   * a step whose two nodes are zero leaves the composite as it is (where the
+//     decay is not negative or NaN), so level size, opacity power and divisions
+//     run for the others alone.
 // Measured: the trace of 1,000,003 samples on the 4M-triangle terrain at
 // L = 9 went from 4.9 to 1.3 ms, 65,536 samples on the room at L = 7 from 0.57
 // to 0.17 ms, every output unchanged.
@@ -103,7 +104,8 @@ __device__ __forceinline__ StepTerm svo_step(const SvoScene& S, const vct_cone_t
     const float level = fminf(fmaxf(fmaxf(K.start_level, raw_level), min_level), (float)(kClipLevels - 1));
     const uint2 v = svo_nodes(S, pos, (uint32_t)floorf(level), (uint32_t)ceilf(level));
     StepTerm t;
-    t.some = (v.x | v.y) != 0u;
+    // (a divisor that vanishes or is NaN turns a step of no opacity into 0 / 0, which ends the march)
+    t.some = (v.x | v.y) != 0u || !(d.occlusion_decay >= 0.0f);
     if (!t.some) return t;
     const float4 a = unpack_rgba8(v.x), b = unpack_rgba8(v.y);
     const float fr = fractf(level);
