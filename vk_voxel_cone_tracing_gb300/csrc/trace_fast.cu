@@ -161,13 +161,21 @@ __device__ __forceinline__ uint32_t morton_key(const vct_surface_sample* __restr
     return spread10(x) | (spread10(y) << 1) | (spread10(z) << 2);
 }
 
-// First bit that the orders are sorted by: cells of eight level-0 voxels, which
-// is three radix passes and leaves a cell's samples in their given order.
-// Whole trace at bit 0 / 6 / 14 (four, three, two passes), us: 4096 samples
-// 53.1 / 50.9 / 51.2, 131,071 in FP16 944 / 932 / 963, 2,073,600 on the hall
-// 8592 / 8602 / 9238.  The batched trace's keys are sorted whole: 64 scenes in one call
-// 15.69 ms, from bit 6 15.96.
+// First bit that the orders are sorted by.  Bit 6 makes cells of eight level-0
+// voxels, which is three radix passes instead of four and leaves a cell's
+// samples in their given order; where many samples share a cell, neighbours'
+// texels are then fetched far apart, which costs more than the pass.  A finer
+// clipmap of the same scene has more cells, so the line goes by samples per R.
+// Whole trace, us, from bit 0 / 6: 4096 samples 53.1 / 50.9; R = 64 room 98,304
+// samples 347 / 347, 200,000 547 / 566, 1,000,000 2125 / 2283; R = 128 room
+// 200,000 683 / 690, 400,000 1203 / 1239, 2,073,600 5563 / 5860; R = 128 hall
+// 262,144 859 / 851, 400,000 1218 / 1215; R = 256 hall 400,000 1874 / 1857,
+// 1,000,000 4254 / 4256, 2,073,600 8460 / 8500.  The batched trace's keys are
+// sorted whole: 64 scenes in one call 15.69 ms, from bit 6 15.96.
 constexpr int kMortonBegin = 6;
+constexpr int64_t kWholeKeysPerR = 3072;
+
+inline int morton_begin(int64_t n, float R) { return (float)n >= (float)kWholeKeysPerR * R ? 0 : kMortonBegin; }
 
 __global__ void k_morton_keys(const vct_surface_sample* __restrict__ s, int64_t n, FastConsts C,
                               uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
@@ -701,10 +709,14 @@ struct FastScratch {
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 static int plan_scratch(int64_t n, void* base, FastScratch& s) {
-    size_t temp_bytes = 0;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                                    (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, kMortonBegin, 30);
-    if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
+    size_t temp_bytes = 0;  // of either sort (morton_begin)
+    for (int begin : {0, kMortonBegin}) {
+        size_t need = 0;
+        cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, need, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                                        (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, begin, 30);
+        if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
+        temp_bytes = need > temp_bytes ? need : temp_bytes;
+    }
     const size_t arr = align256(sizeof(uint32_t) * (size_t)n);
     char* p = (char*)base;
     size_t off = 0;
@@ -866,7 +878,7 @@ int launch_fast(const FastArgs& A, const FastScratch& S, int64_t n, FastShape sh
     VCT_LAUNCH_CHECK();
     size_t tb = S.temp_bytes;
     VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(S.temp, tb, S.keys_in, S.keys_out, S.vals_in, S.order, (int)n,
-                                                 kMortonBegin, 30, st));
+                                                 morton_begin(n, A.P.d.volume_dimension), 30, st));
     // the specular count and the tickets of the specular cones and the diffuse items
     VCT_CUDA_TRY(cudaMemsetAsync(S.spec_count, 0, 3 * sizeof(unsigned int), st));
     const int per_warp = deal_samples_per_warp(n, (int64_t)sms * kDiffuseWarpsPerSm);
