@@ -20,6 +20,7 @@ extern "C" int vct_clipmap_frame(const vct_scene* scene, const vct_frame_desc* f
                                  vct_workspace_s* ws, void* stream) {
     vct::NvtxRange range("vct_clipmap_frame");
     VCT_CHECK_ARG(scene && f && opacity && radiance && ws, "vct_clipmap_frame: null argument");
+    VCT_CHECK_ARG(opacity != radiance, "vct_clipmap_frame: radiance and opacity atlases must differ");
     VCT_CHECK_ARG(!f->shadow_width || shadow_depth, "vct_clipmap_frame: shadow map size given without a buffer");
     VCT_CHECK_ARG(f->inject_mode == VCT_INJECT_DETERMINISTIC || f->inject_mode == VCT_INJECT_ATOMIC,
                   "vct_clipmap_frame: bad injection mode");
