@@ -718,6 +718,7 @@ struct TilePlan {
     const uint32_t* tile_item;  // item of every tile
     uint32_t total;             // tiles
     unsigned int* ticket;       // the next chunk of 32 tiles a coverage warp takes (zeroed per launch)
+    int* err;                   // the atomic injection's error word, in the ticket's slot (the arena may end behind it)
     int group;                  // of the launch: chunk_group
 };
 
@@ -2007,6 +2008,7 @@ static int plan_tiles(RasterArgs& A, vct_workspace_s* ws, size_t& off, TilePlan*
     plan->tile_item = tile_item;
     plan->total = total;
     plan->ticket = ticket;
+    plan->err = (int*)(ticket + 1);
     plan->group = 0;
     return VCT_OK;
 }
@@ -2690,7 +2692,7 @@ extern "C" int vct_inject_radiance(const vct_scene* scene, const vct_clipmap_reg
         rc = plan_tiles(A, ws, off, &plan, st);
         if (rc != VCT_OK) return rc;
         if (plan.total == 0) return VCT_OK;
-        int* err = (int*)((char*)ws->ptr + off);
+        int* err = plan.err;
         VCT_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
         launch_cover<K_INJECT, P_DIRECT>(A, plan, nullptr, nullptr, nullptr, err, st);
         VCT_LAUNCH_CHECK();
