@@ -84,12 +84,13 @@ __device__ __forceinline__ float calc_min_level(const vct_cone_tracing_desc& d, 
     return ceilf(min_level);
 }
 
-// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map.
+// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map.  The texel indices are clamped to just outside it
+// before they become integers: a tap may lie past 2^31 texels, where the index after the last integer is undefined.
 __device__ __forceinline__ float shadow_tap(const float* __restrict__ depth, int W, int H, float s, float t) {
     float u = s * (float)W - 0.5f, v = t * (float)H - 0.5f;
     float fu = floorf(u), fv = floorf(v);
     float a = u - fu, b = v - fv;
-    int i0 = (int)fu, j0 = (int)fv;
+    int i0 = (int)fminf(fmaxf(fu, -2.0f), (float)W), j0 = (int)fminf(fmaxf(fv, -2.0f), (float)H);
     auto at = [&](int i, int j) -> float {
         if (i < 0 || j < 0 || i >= W || j >= H) return 0.0f;
         return __ldg(depth + (int64_t)j * W + i);
@@ -160,8 +161,8 @@ __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp
         if (k == 0) i0 = (int)fu, j0 = (int)fv;
         window = window && fu == (float)i0 + (float)k && fv == (float)j0 + (float)k;
     }
-    // beyond 2^23 texels consecutive indices are no longer distinct floats
-    window = window && (unsigned)(i0 + (1 << 22)) < (1u << 23) && (unsigned)(j0 + (1 << 22)) < (1u << 23);
+    // beyond 2^23 texels consecutive indices are no longer distinct floats (and past 2^31 the conversions saturate)
+    window = window && (unsigned)i0 + (1u << 22) < (1u << 23) && (unsigned)j0 + (1u << 22) < (1u << 23);
     float sum = 0.0f;
     if (window) {
         if (i0 + 4 < 0 || j0 + 4 < 0 || i0 >= W || j0 >= H) return 0.0f;
