@@ -1658,20 +1658,30 @@ __device__ __forceinline__ bool adds_to(uint32_t flags, int f) {
     return (flags & kInjLit) && ((flags & kInjEmissive) || ((flags >> (2 + f / 2)) & 1u) == (uint32_t)(f & 1));
 }
 
-// Runs and lit samples past which a block folds a voxel (k_inject_fold_long).
+// Runs and samples past which a block folds a voxel (k_inject_fold_long).  Both
+// folds ask these two, so that each voxel is folded by one of them: a run holds
+// at most 32 samples, so the samples of kLongVoxelSamples / 32 runs or fewer
+// need no count, and those of more than kLongVoxelRuns runs none either.
 constexpr uint32_t kLongVoxelRuns = 64, kLongVoxelSamples = 192;
+static_assert(kLongVoxelSamples % 32 == 0, "whole runs");
+__device__ __forceinline__ bool counts_samples(uint32_t runs) {
+    return runs > kLongVoxelSamples / 32u && runs <= kLongVoxelRuns;
+}
+// `samples`: of the voxel's runs where counts_samples(runs), else at most kLongVoxelSamples.
+__device__ __forceinline__ bool is_long_voxel(uint32_t runs, uint32_t samples) {
+    return runs > kLongVoxelRuns || samples > kLongVoxelSamples;
+}
 
-// The long voxels: more than kLongVoxelRuns runs, or more than
-// kLongVoxelSamples samples (eight runs hold at most 256).
+// Lists the long voxels.
 template <class Key, class Run>
 __global__ void __launch_bounds__(256) k_inject_long(const FoldArgs<Key, Run> F) {
     const uint32_t voxels = *F.nheads - 1u;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < voxels; v += gridDim.x * blockDim.x) {
         const uint32_t h0 = F.heads[v], h1 = F.heads[v + 1];
         uint32_t sum = 0u;
-        if (h1 - h0 > kLongVoxelSamples / 32u && h1 - h0 <= kLongVoxelRuns)
+        if (counts_samples(h1 - h0))
             for (uint32_t h = h0; h < h1; ++h) sum += (uint32_t)(F.runs[h] & 31u) + 1u;
-        if (h1 - h0 > kLongVoxelRuns || sum > kLongVoxelSamples) F.long_list[atomicAdd(F.nlong, 1u)] = v;
+        if (is_long_voxel(h1 - h0, sum)) F.long_list[atomicAdd(F.nlong, 1u)] = v;
     }
 }
 
@@ -1703,16 +1713,15 @@ __global__ void __launch_bounds__(128) k_inject_fold(const FoldArgs<Key, Run> F)
             key = F.keys[h];
             texel = voxel_texel(key, F.R) + (F.R + 2) * (int64_t)(2 * axis);
         }
-        bool is_long = h1 - h > kLongVoxelRuns;
-        if (__any_sync(FULL, h1 - h > kLongVoxelSamples / 32u && !is_long)) {
-            uint32_t sum = 0u;
-            for (uint32_t r = h + (uint32_t)lg; r < h1 && !is_long; r += (uint32_t)G) sum += (uint32_t)(F.runs[r] & 31u) + 1u;
+        uint32_t samples = 0u;
+        if (__any_sync(FULL, counts_samples(h1 - h))) {
+            if (counts_samples(h1 - h))
+                for (uint32_t r = h + (uint32_t)lg; r < h1; r += (uint32_t)G) samples += (uint32_t)(F.runs[r] & 31u) + 1u;
             __syncwarp();
 #pragma unroll
-            for (int o = 1; o < G; o <<= 1) sum += __shfl_xor_sync(FULL, sum, o);
-            is_long = is_long || sum > kLongVoxelSamples;
+            for (int o = 1; o < G; o <<= 1) samples += __shfl_xor_sync(FULL, samples, o);
         }
-        if (is_long) h1 = h;
+        if (is_long_voxel(h1 - h, samples)) h1 = h;
         const bool mine = h < h1;  // a voxel of the warp's, not a long one
         AvgCell even = avg_cell(0u), odd = even;
         if (!F.lit && mine) {
