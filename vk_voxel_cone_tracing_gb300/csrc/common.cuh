@@ -83,7 +83,7 @@ int wrap_border_r8(uint8_t* atlas, int R, cudaStream_t st);
 int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const vct_clipmap_region regions[6],
                         uint32_t due, const vct_clipmap_region* slabs, const int32_t* slab_levels, int nslabs,
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
-                        cudaSurfaceObject_t mirror, FrameBits* bits, cudaStream_t st);
+                        cudaSurfaceObject_t mirror, cudaStream_t st);
 
 // ---------------------------------------------------------------- errors
 void set_error(const std::string& msg);

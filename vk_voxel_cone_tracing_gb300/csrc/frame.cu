@@ -65,9 +65,8 @@ extern "C" int vct_clipmap_frame(const vct_scene* scene, const vct_frame_desc* f
         // coverage count sharing one coverage pass and the clears and
         // copy-alpha passes done from voxel bits (same results as the passes
         // below)
-        vct::FrameBits bits;
         return vct::frame_raster_passes(scene, f, regions, due, slabs, slab_levels, nslabs, opacity, radiance,
-                                        shadow_depth, ws, mirror, &bits, st);
+                                        shadow_depth, ws, mirror, st);
     } else {
         if (!toroidal) {
             // VoxelizationPass (full revoxelisation every frame, VoxelizationPass.cpp:79-125)

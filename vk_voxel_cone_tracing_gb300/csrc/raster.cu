@@ -2833,7 +2833,7 @@ static int join_side(vct_workspace_s* ws, cudaStream_t side, cudaStream_t st) {
 int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const vct_clipmap_region regions[6],
                         uint32_t due, const vct_clipmap_region* slabs, const int32_t* slab_levels, int nslabs,
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
-                        cudaSurfaceObject_t mirror, FrameBits* bits_out, cudaStream_t st) {
+                        cudaSurfaceObject_t mirror, cudaStream_t st) {
     const int R = f->clipmap_resolution;
     int rc;
     const bool toroidal = nslabs >= 0;
@@ -2851,7 +2851,7 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
         VCT_CUDA_TRY(cudaMalloc(&ws->aux, bm_bytes));
         ws->aux_bytes = bm_bytes;
     }
-    FrameBits& B = *bits_out;
+    FrameBits B;
     B.lit = (uint32_t*)ws->aux;
     B.opaque = toroidal ? nullptr : (uint32_t*)((char*)ws->aux + map_bytes);
     B.nonzero = toroidal ? nullptr : (uint32_t*)((char*)ws->aux + 2 * map_bytes);
