@@ -84,13 +84,13 @@ __device__ __forceinline__ float calc_min_level(const vct_cone_tracing_desc& d, 
     return ceilf(min_level);
 }
 
-// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map.  The texel indices are clamped to just outside it
-// before they become integers: a tap may lie past 2^31 texels, where the index after the last integer is undefined.
+// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map.  The texel indices are clamped, outside any map, before
+// they become integers: a tap may lie past 2^31 texels, where the index after the last integer is undefined.
 __device__ __forceinline__ float shadow_tap(const float* __restrict__ depth, int W, int H, float s, float t) {
     float u = s * (float)W - 0.5f, v = t * (float)H - 0.5f;
     float fu = floorf(u), fv = floorf(v);
     float a = u - fu, b = v - fv;
-    int i0 = (int)fminf(fmaxf(fu, -2.0f), (float)W), j0 = (int)fminf(fmaxf(fv, -2.0f), (float)H);
+    int i0 = (int)fminf(fmaxf(fu, -2.0f), 0x1p30f), j0 = (int)fminf(fmaxf(fv, -2.0f), 0x1p30f);
     auto at = [&](int i, int j) -> float {
         if (i < 0 || j < 0 || i >= W || j >= H) return 0.0f;
         return __ldg(depth + (int64_t)j * W + i);
