@@ -1,4 +1,5 @@
 // capi.cu -- error state, version, and the host-side pieces of the C ABI.
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -22,6 +23,18 @@ int cuda_fail(cudaError_t e, const char* what) {
     // not report it again; a sticky error stays and is reported by every later call
     cudaGetLastError();
     return VCT_E_CUDA;
+}
+
+int sm_count() {
+    static std::atomic<int> counts[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+    int c = counts[dev].load(std::memory_order_relaxed);
+    if (!c) {
+        if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0) c = 152;
+        counts[dev].store(c, std::memory_order_relaxed);
+    }
+    return c;
 }
 
 }  // namespace vct

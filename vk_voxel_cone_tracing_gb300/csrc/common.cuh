@@ -75,7 +75,7 @@ int wrap_border_r8(uint8_t* atlas, int R, cudaStream_t st);
 // voxelisation, mips and border, shadow depth, injection, and the due radiance
 // levels' copy-alpha and mips, mirrored into `mirror` (0: none).
 // The radiance levels due are not cleared: the fold starts their texels from
-// zero, stores all faces of each voxel it lights and marks it in *bits, and the
+// zero, stores all faces of each voxel it lights and marks its bit, and the
 // passes after it take unmarked voxels as zero rgb -- the cleared result.
 // With nslabs >= 0 the opacity atlas is updated toroidally: only the listed
 // slabs are cleared and revoxelised (levels with a whole-region slab in
@@ -84,6 +84,10 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
                         uint32_t due, const vct_clipmap_region* slabs, const int32_t* slab_levels, int nslabs,
                         uint32_t* opacity, uint32_t* radiance, float* shadow_depth, vct_workspace_s* ws,
                         cudaSurfaceObject_t mirror, cudaStream_t st);
+
+// SMs of the current device (152 where it cannot be asked), for the rules that
+// split work by how much fills the chip.
+int sm_count();
 
 // ---------------------------------------------------------------- errors
 void set_error(const std::string& msg);

@@ -2178,13 +2178,14 @@ static int inject_group_and_fold(const RasterArgs& I, const InjectState& S, uint
         VCT_CUDA_TRY(cudaStreamWaitEvent(side, ws->fork2, 0));
     }
     cudaStream_t lst = side ? side : st;
+    const int sms = sm_count();
     k_inject_long<Key, Run><<<grid_of(runs, 256), 256, 0, lst>>>(F);
     VCT_LAUNCH_CHECK();
-    k_inject_fold_long<Key, Run, 1024><<<152, 1024, 0, lst>>>(F);
+    k_inject_fold_long<Key, Run, 1024><<<sms, 1024, 0, lst>>>(F);
     VCT_LAUNCH_CHECK();
-    k_inject_fold_long<Key, Run, 256><<<152 * 8, 256, 0, lst>>>(F);
+    k_inject_fold_long<Key, Run, 256><<<sms * 8, 256, 0, lst>>>(F);
     VCT_LAUNCH_CHECK();
-    k_inject_fold<Key, Run><<<grid_of((int64_t)runs * 4, 128, 152 * 64), 128, 0, st>>>(F);
+    k_inject_fold<Key, Run><<<grid_of((int64_t)runs * 4, 128, sms * 64), 128, 0, st>>>(F);
     VCT_LAUNCH_CHECK();
     if (side) {
         VCT_CUDA_TRY(cudaEventRecord(ws->join2, side));

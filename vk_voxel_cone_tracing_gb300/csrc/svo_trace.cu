@@ -360,13 +360,13 @@ extern "C" int vct_svo_cone_trace(const vct_cone_tracing_desc* desc, const vct_c
         ExactPlan plan;
         rc = exact_plan(smp, m, P.d, &plan, st);
         if (rc != VCT_OK) return rc;
-        const int per_warp = deal_samples_per_warp(m, 152 * kSvoWarpsPerSm);
+        const int sms = sm_count(), per_warp = deal_samples_per_warp(m, (int64_t)sms * kSvoWarpsPerSm);
         const int64_t gd = (m + (int64_t)per_warp * kSvoWarps - 1) / ((int64_t)per_warp * kSvoWarps);
-        k_svo_diffuse<<<(int)(gd > 152 * 8 ? 152 * 8 : gd), 32 * kSvoWarps, 0, st>>>(
+        k_svo_diffuse<<<(int)(gd > sms * 8 ? sms * 8 : gd), 32 * kSvoWarps, 0, st>>>(
             P, S, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, plan.spec_count + 2, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            const int64_t gs = (m * kMaxConeGroup + 127) / 128, full = 152 * kSvoSpecWarpsPerSm / 4;
+            const int64_t gs = (m * kMaxConeGroup + 127) / 128, full = (int64_t)sms * kSvoSpecWarpsPerSm / 4;
             k_svo_specular<<<(int)(gs > full ? full : gs), 128, 0, st>>>(
                 P, S, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, plan.spec_count + 1);
             e = cudaGetLastError();

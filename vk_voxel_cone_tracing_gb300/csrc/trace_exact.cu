@@ -367,13 +367,13 @@ static int launch_exact(const TraceParams& P, const Atlas& T, const vct_surface_
         if (rc != VCT_OK) return rc;
         unsigned int* spec_ticket = plan.spec_count + 1;
         unsigned int* diff_ticket = plan.spec_count + 2;
-        const int per_warp = deal_samples_per_warp(m, 152 * kExactDiffuseWarpsPerSm);
+        const int sms = sm_count(), per_warp = deal_samples_per_warp(m, (int64_t)sms * kExactDiffuseWarpsPerSm);
         const int64_t gdw = (m + (int64_t)per_warp * kExactWarps - 1) / ((int64_t)per_warp * kExactWarps);
-        k_exact_diffuse<<<(int)(gdw > 152 * 16 ? 152 * 16 : gdw), 32 * kExactWarps, 0, st>>>(
+        k_exact_diffuse<<<(int)(gdw > sms * 16 ? sms * 16 : gdw), 32 * kExactWarps, 0, st>>>(
             P, C, T, smp, m, plan.order, dout + 4 * off, sout + 4 * off, cone_steps, diff_ticket, per_warp);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
-            const int64_t gl = (m * kMaxConeGroup + 127) / 128, full = 152 * kExactSpecWarpsPerSm / 4;
+            const int64_t gl = (m * kMaxConeGroup + 127) / 128, full = (int64_t)sms * kExactSpecWarpsPerSm / 4;
             k_exact_specular<<<(int)(gl > full ? full : gl), 128, 0, st>>>(
                 P, C, T, smp, plan.spec_list, plan.spec_count, sout + 4 * off, cone_steps, spec_ticket);
             e = cudaGetLastError();

@@ -840,18 +840,6 @@ struct FastShape {
     int diffuse_per_sm = 8, specular_per_sm = 64;
 };
 
-int sm_count() {
-    static int counts[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
-    if (!counts[dev]) {
-        int c = 0;
-        if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0) c = 152;
-        counts[dev] = c;
-    }
-    return counts[dev];
-}
-
 // Shapes chosen by vct_cone_trace_fast_autotune, per (device, log2 R).
 std::mutex g_shape_mutex;
 FastShape g_shapes[8][11];
@@ -1173,6 +1161,7 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
     unsigned int* spec_count = reinterpret_cast<unsigned int*>(b + L.spec_count);
     int jb = 0;
     while ((1 << jb) < kBatchJobs) ++jb;
+    const int sms = sm_count();
     std::vector<BatchTable> tables((job_count + kBatchJobs - 1) / kBatchJobs);
     for (size_t c = 0; c < tables.size(); ++c) {
         BatchTable& T = tables[c];
@@ -1204,7 +1193,7 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
         T.bases[T.njobs] = pos;
         if (pos == 0) continue;
         const int64_t n = pos;
-        const int g256 = (int)((n + 255) / 256 > 152 * 32 ? 152 * 32 : (n + 255) / 256);
+        const int g256 = (int)((n + 255) / 256 > sms * 32 ? sms * 32 : (n + 255) / 256);
         k_batch_keys<<<g256, 256, 0, st>>>(T, pos, keys_in, vals_in);
         VCT_LAUNCH_CHECK();
         size_t tb = L.temp_bytes;
@@ -1213,7 +1202,7 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
         VCT_CUDA_TRY(cudaMemsetAsync(spec_count, 0, 2 * sizeof(unsigned int), st));  // count and cone ticket
         if (pos < kBatchSpecOrdered) {
             const int64_t gk = (n + kSpecListChunk - 1) / kSpecListChunk;
-            k_batch_spec_list<<<(int)(gk > 152 * 8 ? 152 * 8 : gk), kSpecListBlock, 0, st>>>(T, pos, order, spec_list,
+            k_batch_spec_list<<<(int)(gk > sms * 8 ? sms * 8 : gk), kSpecListBlock, 0, st>>>(T, pos, order, spec_list,
                                                                                            spec_count);
             VCT_LAUNCH_CHECK();
         } else {
@@ -1228,12 +1217,12 @@ extern "C" int vct_cone_trace_fast_batch(const vct_trace_job* jobs, int32_t job_
             k_batch_spec_order<<<g256, 256, 0, st>>>(words, order, masks, offs, spec_list, spec_count);
             VCT_LAUNCH_CHECK();
         }
-        const int per_warp = deal_samples_per_warp(n, 152 * kDiffuseWarpsPerSm);
+        const int per_warp = deal_samples_per_warp(n, (int64_t)sms * kDiffuseWarpsPerSm);
         const int64_t gd = (n + (int64_t)per_warp * kWarpsPerBlock - 1) / ((int64_t)per_warp * kWarpsPerBlock);
-        k_batch_diffuse<<<(int)(gd > 152 * 8 ? 152 * 8 : gd), 256, 0, st>>>(T, pos, order, per_warp);
+        k_batch_diffuse<<<(int)(gd > sms * 8 ? sms * 8 : gd), 256, 0, st>>>(T, pos, order, per_warp);
         VCT_LAUNCH_CHECK();
         const int64_t gw = (n * 32 + 255) / 256;
-        k_batch_specular<<<(int)(gw > 152 * 64 ? 152 * 64 : gw), 256, 0, st>>>(T, spec_list, spec_count,
+        k_batch_specular<<<(int)(gw > sms * 64 ? sms * 64 : gw), 256, 0, st>>>(T, spec_list, spec_count,
                                                                                 spec_count + 1);
         VCT_LAUNCH_CHECK();
     }
