@@ -1108,15 +1108,26 @@ __device__ __forceinline__ uint32_t chunk_tile(uint32_t ch, uint32_t nchunks, in
 // hundreds in a row) and a few on a chunk of small triangles, and the longest
 // chunk was the kernel's time: 85 % of the SM cycles idle on a 34k-triangle
 // room.  Chunks whose tiles come from all over the list are alike; many tiles
-// need less of it, and consecutive ones share their loads.  Measured (us at 32
-// / 8 / 4 / 2 consecutive): opacity + count of 206k tiles 322 / - / 92 / 68,
-// emission 209 / - / 62 / 44; octree count of 4.3M tiles 1202 / - / 1115 /
-// 1142; opacity + count of 5.6M tiles 1714 / - / 1755 / 1773.  The one-sample
-// passes (shadow, G-buffer) have cheap full tiles and keep 32: 114 against 122
-// / 127 us at 280k tiles.
+// need less of it, and consecutive ones share their loads.  Measured, count and
+// emission together, us at 1 / 2 / 4 / 8 / 32 consecutive tiles:
+//   frame   203,843 tiles   65 /  83 / 122 / 193 / 451
+//           282,602         76 /  92 / 139 / 219 / 606
+//           398,685         93 / 100 / 142 / 218 / 630
+//           843,680        167 / 162 / 177 / 239 / 639
+//         1,400,728        256 / 250 / 246 / 280 / 647
+//         2,152,243        536 / 519 / 517 / 511 / 970
+//         4,756,939       1102 / 1084 / 1074 / 1056 / 1186
+//   octree  106,111        242 / 260 / 282 / 290 / 586
+//           417,302        186 / 175 / 175 / 180 / 246
+//           780,370        604 / 591 / 588 / 597 / 632
+//         1,802,536       1027 / 996 / 985 / 983 / 1042
+//         4,300,000       1293 / 1272 / 1257 / 1265 / 1314
+// (between 2^18 and 2^19 the frame would rather have 1, the octree 2 or 4).  The
+// one-sample passes (shadow, G-buffer) have cheap full tiles, whose time this
+// does not change (54 us at any of the five, 322,395 tiles): they keep 32.
 static int chunk_group(bool one_sample, uint32_t tiles) {
     if (one_sample) return 5;
-    return tiles < (1u << 18) ? 0 : (tiles < (1u << 20) ? 1 : 3);
+    return tiles < (1u << 18) ? 0 : (tiles < (1u << 20) ? 1 : (tiles < (1u << 21) ? 2 : 3));
 }
 
 // Coverage kernels.  A warp takes 32 8x8 tiles of (triangle, level) items
@@ -2858,11 +2869,14 @@ int frame_raster_passes(const vct_scene* scene, const vct_frame_desc* f, const v
     B.nonzero = toroidal ? nullptr : (uint32_t*)((char*)ws->aux + 2 * map_bytes);
     VCT_CUDA_TRY(cudaMemsetAsync(ws->aux, 0, bm_bytes, st));
     // Two stretches run on the side stream (with its own workspace), beside
-    // main-stream work they share no buffer with: the shadow pass beside the
-    // opacity clear, voxelisation and injection count / emission (the shadow
-    // map is read only by the injection's shading, after the join), and the
-    // opacity mips + border wrap beside the shading, sort and fold.  The
-    // results are those of the serial order.
+    // main-stream work they share no written buffer with: the shadow pass
+    // beside the opacity voxelisation (with the toroidal update's slab clear)
+    // and injection count / emission (the shadow map is read only by the
+    // injection's shading, after the join), and the opacity fill, mips and
+    // border wrap beside the shading, sort, fold and, in a full update, the
+    // radiance fill (both fills read the voxel bits).  The long voxels' folds
+    // run on the second side stream beside the others.  The results are those
+    // of the serial order.
     cudaStream_t side = side_stream(ws);
     cudaStream_t sst = side ? side : st;  // the shadow pass's stream
     vct_workspace_s* sws = side ? ws->side_ws : ws;
