@@ -11,7 +11,7 @@
 // due level goes to the atlas and to the texture.
 // Measured, R = 256 hall frame: k_opacity_fill 0.35 ms (7.0 TB/s) where a clear,
 // scattered six-face stores and their write-backs were; k_radiance_fill 1.16 ms
-// with the texture (4.7 TB/s), 0.72 ms without, and the five k_radiance_mip
+// with the texture (4.2 TB/s), 0.72 ms without (3.4), and the five k_radiance_mip
 // 0.50 ms, where copy-alpha and the fused copy-alpha + mip passes took 0.37 +
 // 2.24 ms (they waited for their loads: DRAM 42 % busy).  The frame 8.59 ->
 // 7.72 ms.  Texture stores of 16 bytes cost 0.44 ms a frame, the 4-byte ones

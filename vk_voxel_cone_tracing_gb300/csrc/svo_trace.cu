@@ -9,11 +9,12 @@
 //
 // Work layout: the exact clipmap trace's plan (samples in the coherent order;
 // the diffuse cones of a warp's samples dealt to its lanes, trace_deal.cuh;
-// the specular cones one per lane over a list grouped by aperture), instead
-// of one thread marching a sample's 17 cones.  The march is bound by its own
-// arithmetic (the pool stays in L2, and most of the box is empty space that a
-// descent leaves after a node or two), so each step computes only what its
-// result needs, every needed value being the shader expression's bit for bit:
+// the specular cones over a list grouped by aperture, one to eight lanes to a
+// cone), instead of one thread marching a sample's 17 cones.  The march is
+// bound by its own arithmetic (the pool stays in L2, and most of the box is
+// empty space that a descent leaves after a node or two), so each step computes
+// only what its result needs, every needed value being the shader expression's
+// bit for bit:
 //   * both levels' nodes come from one descent (the coarser is an ancestor),
 //     child slots straight from the cell's bits, a node read as one 8 bytes;
 //   * the cell is a fused multiply-add and a floor per axis, the shader's

@@ -308,10 +308,10 @@ __device__ __forceinline__ void write_outputs(const TraceParams& p, const GSampl
 }
 
 // A coherent processing order of G-buffer samples: radix-sorted by normal
-// class (6 bits, octahedral 8 x 8) and then by the Morton code of the
-// position on a grid of two level-0 voxels per cell around the volume centre
-// (10 bits per axis, 64-bit keys).  Per-sample results do not depend on the processing
-// order, so the per-thread kernels walk this permutation: a warp's lanes skip
+// class (6 bits, octahedral 8 x 8) and then by the upper 26 bits of the Morton
+// code of the position on a grid of two level-0 voxels per cell around the
+// volume centre (10 bits per axis; 32-bit keys).  Per-sample results do not
+// depend on the processing order, so the kernels walk this permutation: a warp's lanes skip
 // the same diffuse cones and their texel fetches (and the adjoint's gradient
 // atomics) land on neighbouring cache lines.  Allocates its buffers
 // stream-ordered: `*block` is freed with cudaFreeAsync after the last kernel

@@ -1,7 +1,7 @@
 // trace_deal.cuh -- the diffuse half of voxelConeTracing.frag's main()
-// (:143-190, 258-293) for one warp of 32 samples, shared by the texture form
-// (trace_fast.cu) and the exact FP32 forms (trace_exact.cu), generic in how
-// one cone is marched.
+// (:143-190, 258-293) for the 4 to 32 samples of a warp item, shared by the
+// texture form (trace_fast.cu), the exact FP32 forms (trace_exact.cu) and the
+// octree (svo_trace.cu), generic in how one cone is marched and a sample ended.
 //
 // The (sample, cone) pairs with cos >= 0 of the warp's samples (up to 32) are
 // dealt to the 32 lanes in rounds, cone-major (lane k of a round takes the k-th

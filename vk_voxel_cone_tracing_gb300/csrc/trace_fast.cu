@@ -833,7 +833,7 @@ namespace {
 
 // Launch shape of the fast trace: the grids of the diffuse and specular
 // kernels in blocks (of 256 threads) per SM.  Result-neutral: both kernels
-// are grid-stride loops in which a sample's diffuse item and a specular cone
+// are loops over the work in which a sample's diffuse item and a specular cone
 // get the same arithmetic whichever warp takes them, and the step counter is
 // an integer sum.
 struct FastShape {

@@ -430,7 +430,7 @@ extern "C" int vct_cone_trace_backward(const vct_cone_tracing_desc* desc, const 
     if (rc != VCT_OK) return rc;
     cudaStream_t st = as_stream(stream);
     const int nc = desc->enable_32_cones ? 32 : 16;
-    // grids of resident blocks (grid-stride loops): the record scratch holds one block per warp of the grid
+    // grids of resident blocks (their warps take work by tickets): the record scratch holds one block per warp
     int dev = 0, sms = 0, occ_d = 0, occ_s = 0;
     VCT_CUDA_TRY(cudaGetDevice(&dev));
     VCT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
