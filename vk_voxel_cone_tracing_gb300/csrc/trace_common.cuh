@@ -84,13 +84,12 @@ __device__ __forceinline__ float calc_min_level(const vct_cone_tracing_desc& d, 
     return ceilf(min_level);
 }
 
-// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map.  The texel indices are clamped, outside any map, before
-// they become integers: a tap may lie past 2^31 texels, where the index after the last integer is undefined.
+// One bilinear CLAMP_TO_BORDER(0) tap of the D32 shadow map, within 2^31 texels of it.
 __device__ __forceinline__ float shadow_tap(const float* __restrict__ depth, int W, int H, float s, float t) {
     float u = s * (float)W - 0.5f, v = t * (float)H - 0.5f;
     float fu = floorf(u), fv = floorf(v);
     float a = u - fu, b = v - fv;
-    int i0 = (int)fminf(fmaxf(fu, -2.0f), 0x1p30f), j0 = (int)fminf(fmaxf(fv, -2.0f), 0x1p30f);
+    int i0 = (int)fu, j0 = (int)fv;
     auto at = [&](int i, int j) -> float {
         if (i < 0 || j < 0 || i >= W || j >= H) return 0.0f;
         return __ldg(depth + (int64_t)j * W + i);
@@ -175,6 +174,10 @@ __device__ __forceinline__ float calc_visibility(const TraceParams& p, float3 wp
             });
         return sum * 0.0625f;
     }
+    // past 2^30 texels no tap meets the map (and past 2^31 the index after a tap's is no integer): zero, NaN where the
+    // position is infinite
+    if ((unsigned)i0 + (1u << 30) >= (1u << 31) || (unsigned)j0 + (1u << 30) >= (1u << 31))
+        return (a[0] + b[0]) * 0.0f;
     for (int yi = 0; yi < 4; ++yi)
         for (int xi = 0; xi < 4; ++xi) {
             float ox = -1.5f + (float)xi, oy = -1.5f + (float)yi;
