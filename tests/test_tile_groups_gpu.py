@@ -1,4 +1,4 @@
-"""The octree's fragment list where chunks take eight consecutive tiles (2^21 tiles and more) and four (from 2^20):
+"""The octree's fragment list where chunks take eight consecutive tiles (3 x 2^19 tiles and more) and four (from 2^20):
 the list of a scene is the list of its first triangles followed by that of the rest."""
 import copy
 

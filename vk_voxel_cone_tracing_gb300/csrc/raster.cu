@@ -1122,12 +1122,14 @@ __device__ __forceinline__ uint32_t chunk_tile(uint32_t ch, uint32_t nchunks, in
 //           780,370        604 / 591 / 588 / 597 / 632
 //         1,802,536       1027 / 996 / 985 / 983 / 1042
 //         4,300,000       1293 / 1272 / 1257 / 1265 / 1314
-// (between 2^18 and 2^19 the frame would rather have 1, the octree 2 or 4).  The
-// one-sample passes (shadow, G-buffer) have cheap full tiles, whose time this
-// does not change (54 us at any of the five, 322,395 tiles): they keep 32.
+// (between 2^18 and 2^19 the frame would rather have 1, the octree 2 or 4), and
+// whole frames of the hall at R = 64 with 4 / 8: 1.14 M tiles 635 / 671, 1.52 M
+// 715 / 729, 1.90 M 801 / 789 (R = 256: 1931 / 1991, 2052 / 2077, 2201 / 2186).
+// The one-sample passes (shadow, G-buffer) have cheap full tiles, whose time
+// this does not change (54 us at any of the five, 322,395 tiles): they keep 32.
 static int chunk_group(bool one_sample, uint32_t tiles) {
     if (one_sample) return 5;
-    return tiles < (1u << 18) ? 0 : (tiles < (1u << 20) ? 1 : (tiles < (1u << 21) ? 2 : 3));
+    return tiles < (1u << 18) ? 0 : (tiles < (1u << 20) ? 1 : (tiles < (3u << 19) ? 2 : 3));
 }
 
 // Coverage kernels.  A warp takes 32 8x8 tiles of (triangle, level) items
