@@ -512,9 +512,9 @@ def run_ours(args, world, rank, local):
                    "sample": f"first {ncpu} of {n} samples ({st} cone samples, {dt:.1f} s) traced by the FP32 C++ "
                              "restatement on the same clipmap"}
         # kernels launched per trace step: Morton keys, cub radix sort (histogram, exclusive sum, 4 onesweep passes
-        # over the whole keys, 3 with fewer than 3072 R samples), specular list, diffuse, specular (the texture
-        # refresh is a memcpy, not a kernel)
-        launches = 1 if tex is None else (10 if n >= 3072 * R else 9)
+        # over the whole keys from 3072 R samples on at R > 128, else 3), specular list, diffuse, specular (the
+        # texture refresh is a memcpy, not a kernel)
+        launches = 1 if tex is None else (10 if R > 128 and n >= 3072 * R else 9)
         line = {
             "metric": METRIC, "value": value, "unit": "cone samples/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",

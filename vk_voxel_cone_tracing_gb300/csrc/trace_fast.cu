@@ -161,21 +161,33 @@ __device__ __forceinline__ uint32_t morton_key(const vct_surface_sample* __restr
     return spread10(x) | (spread10(y) << 1) | (spread10(z) << 2);
 }
 
-// First bit that the orders are sorted by.  Bit 6 makes cells of eight level-0
-// voxels, which is three radix passes instead of four and leaves a cell's
-// samples in their given order; where many samples share a cell, neighbours'
-// texels are then fetched far apart, which costs more than the pass.  A finer
-// clipmap of the same scene has more cells, so the line goes by samples per R.
-// Whole trace, us, from bit 0 / 6: 4096 samples 53.1 / 50.9; R = 64 room 98,304
-// samples 347 / 347, 200,000 547 / 566, 1,000,000 2125 / 2283; R = 128 room
-// 200,000 683 / 690, 400,000 1203 / 1239, 2,073,600 5563 / 5860; R = 128 hall
-// 262,144 859 / 851, 400,000 1218 / 1215; R = 256 hall 400,000 1874 / 1857,
-// 1,000,000 4254 / 4256, 2,073,600 8460 / 8500.  The batched trace's keys are
-// sorted whole: 64 scenes in one call 15.69 ms, from bit 6 15.96.
-constexpr int kMortonBegin = 6;
-constexpr int64_t kWholeKeysPerR = 3072;
+// The bits that an order is sorted by: 24 of the key's 30 are three radix passes
+// instead of four.  Bits 6 to 29 make cells of eight level-0 voxels and leave a
+// cell's samples in their given order; where many samples of no order share a
+// cell, neighbours' texels are then fetched far apart, so from some samples per
+// R on (a finer clipmap of the same scene has more cells) the low bits are
+// sorted too.  Up to R = 128 the high ones then go instead: the order repeats
+// every 256 voxels, which is 32 units of the scene or more; at R = 256 it is 16,
+// and the halves of a hall mixed so cost more than a pass.
+// Whole trace, us, from bit 6 / bits 0 to 23 / all: 4096 samples 50.9 / - / 53.1;
+// R = 64 room 131,072 samples 416 / 397 / 411, 1,000,000 2280 / 2109 / 2122;
+// R = 64 hall 131,072 403 / 398 / -; R = 128 room 262,144 864 / 835 / 848,
+// 1,200,000 3432 / 3258 / 3267; R = 128 hall 262,144 848 / 843 / 859; R = 256 room
+// 400,000 1829 / - / 1817, hall 400,000 1857 / - / 1874, 800,000 3519 / 3689 /
+// 3538, 2,073,600 8600 / 8930 / 8592; rendered frame of the hall at
+// R = 64, 1280 x 720 pixels in their order, 2230 / 2215 / 2231.  The batched
+// trace's keys are sorted whole: 64 scenes in one call 15.69 ms, from bit 6
+// 15.96.
+constexpr int kMortonBits = 30, kMortonBegin = 6;
 
-inline int morton_begin(int64_t n, float R) { return (float)n >= (float)kWholeKeysPerR * R ? 0 : kMortonBegin; }
+struct KeyBits {
+    int begin, end;
+};
+inline KeyBits key_bits(int64_t n, float R) {
+    if (R <= 128.0f && (float)n >= 2048.0f * R) return {0, kMortonBits - kMortonBegin};
+    if (R > 128.0f && (float)n >= 3072.0f * R) return {0, kMortonBits};
+    return {kMortonBegin, kMortonBits};
+}
 
 __global__ void k_morton_keys(const vct_surface_sample* __restrict__ s, int64_t n, FastConsts C,
                               uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
@@ -709,11 +721,11 @@ struct FastScratch {
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 static int plan_scratch(int64_t n, void* base, FastScratch& s) {
-    size_t temp_bytes = 0;  // of either sort (morton_begin)
+    size_t temp_bytes = 0;  // of any of the sorts (key_bits)
     for (int begin : {0, kMortonBegin}) {
         size_t need = 0;
         cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, need, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                                        (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, begin, 30);
+                                                        (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, begin, kMortonBits);
         if (e != cudaSuccess) return cuda_fail(e, "cub::DeviceRadixSort::SortPairs (size query)");
         temp_bytes = need > temp_bytes ? need : temp_bytes;
     }
@@ -865,8 +877,9 @@ int launch_fast(const FastArgs& A, const FastScratch& S, int64_t n, FastShape sh
     k_morton_keys<<<grid_keys, block, 0, st>>>(A.samples, n, A.C, S.keys_in, S.vals_in);
     VCT_LAUNCH_CHECK();
     size_t tb = S.temp_bytes;
+    const KeyBits bits = key_bits(n, A.P.d.volume_dimension);
     VCT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(S.temp, tb, S.keys_in, S.keys_out, S.vals_in, S.order, (int)n,
-                                                 morton_begin(n, A.P.d.volume_dimension), 30, st));
+                                                 bits.begin, bits.end, st));
     // the specular count and the tickets of the specular cones and the diffuse items
     VCT_CUDA_TRY(cudaMemsetAsync(S.spec_count, 0, 3 * sizeof(unsigned int), st));
     const int per_warp = deal_samples_per_warp(n, (int64_t)sms * kDiffuseWarpsPerSm);
